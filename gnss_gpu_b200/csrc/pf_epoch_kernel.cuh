@@ -87,15 +87,28 @@ __device__ __forceinline__ void grid_barrier(const EngineDev& e, unsigned* bar, 
   __syncthreads();
 }
 
-// Named CTA barriers over all kThreads threads: arrive without waiting,
-// or wait for the barrier to complete.
-template <int ID>
-__device__ __forceinline__ void named_arrive() {
-  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(kThreads) : "memory");
+// Hand-over of the warps' statistics rows to the warp that merges a tile
+// (shared-memory counters, release / acquire at CTA scope).
+__device__ __forceinline__ void cta_red_release(unsigned* p) {
+  asm volatile("red.release.cta.shared.add.u32 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
 }
-template <int ID>
-__device__ __forceinline__ void named_sync() {
-  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(kThreads) : "memory");
+__device__ __forceinline__ void cta_st_release(unsigned* p, unsigned v) {
+  asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+}
+// Waits until *p has reached `want` (counters only grow).  The other warps of
+// the CTA always run on, so the wait ends; the limit only guards against a
+// fault elsewhere.
+__device__ __forceinline__ void cta_wait_reach(const EngineDev& e, const unsigned* p, unsigned want) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  for (unsigned spins = 0;; ++spins) {
+    unsigned v;
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    if ((int)(v - want) >= 0) return;
+    if (spins > (1u << 24)) {
+      atomicOr(e.err, ERR_BARRIER_TIMEOUT);
+      return;
+    }
+  }
 }
 
 // Reads through L2 of control-block fields that another CTA wrote before a
@@ -327,6 +340,41 @@ __device__ __forceinline__ void epoch_sys_offspring(const EngineDev& e, int cb, 
   }
 }
 
+// One warp merges the warp rows of tile t (the CTA's j-th) into the tile row
+// and, when the filter may resample, forms the tile level of its tiled
+// integer CDF.  The order of the sums is fixed, so the merging warp does not
+// matter.
+constexpr int kRowBufs = 4;   // row buffers
+constexpr int kMergeLag = 2;  // tiles between writing and merging the rows
+template <int NV, int NW>
+__device__ __forceinline__ void merge_rows(const EngineDev& e, int t, int j, const float (*s_wrow)[NW][17],
+                                           const double (*s_wq)[NW], const unsigned* s_rows, unsigned* s_merged) {
+  const int lane = threadIdx.x & 31, b = j % kRowBufs;
+  cta_wait_reach(e, s_rows + b, (unsigned)(NW * (j / kRowBufs + 1)));
+  const float (*wr)[17] = s_wrow[b];
+  const float mw = lane < NW ? wr[lane][0] : -INFINITY;
+  const float tm = warp_max(mw);
+  float acc = 0.f;
+  if (lane < NV && tm > -INFINITY) {
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      const float m = wr[w][0];
+      if (m > -INFINITY) {
+        float sc = exp2f((m - tm) * 1.4426950408889634f);
+        if (lane == 1) sc *= sc;
+        acc = fmaf(sc, wr[w][1 + lane], acc);
+      }
+    }
+  }
+  float* row = e.part + (size_t)t * kPartStride;
+  if (lane < NV) row[1 + lane] = acc;
+  if (lane == 0) row[0] = tm;
+  const double S = lane < NW ? s_wq[b][lane] : 0.0;
+  if (__shfl_sync(0xffffffffu, S, 0) >= 0.0) sys_tile_scale(e, t, S, mw, tm);
+  __syncwarp();
+  if (lane == 0) cta_st_release(s_merged + b, (unsigned)(j / kRowBufs + 1));
+}
+
 #ifndef PF_EPOCH_MINB
 #define PF_EPOCH_MINB 2  // resident CTAs per SM the epoch kernel is compiled for
 #endif
@@ -339,11 +387,12 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
   __shared__ __align__(16) float2 s_sat[kStride * PF_MAX_SATS];
   __shared__ int s_grp[PF_MAX_CLK + 1];
   __shared__ unsigned char s_clk[PF_MAX_SATS];
-  __shared__ float s_wrow[2][kWarps][17];
+  __shared__ float s_wrow[kRowBufs][kWarps][17];
   __shared__ float s_maxtmp[kWarps];
   __shared__ double s_dred[kWarps * 16];
   __shared__ unsigned long long s_u64[2 * kWarps];
-  __shared__ double s_wq[2][kWarps];  // per-warp sums of the tiled integer CDF
+  __shared__ double s_wq[kRowBufs][kWarps];  // per-warp sums of the tiled integer CDF
+  __shared__ unsigned s_rows[kRowBufs], s_merged[kRowBufs];  // rows written, tiles merged (counts per buffer)
   __shared__ int s_dec_f, s_dec_rs;  // the filter this CTA owns in phase 2 and its decision
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -353,6 +402,7 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
   // acquire here would hold every later load of the CTA behind it.
   unsigned gen = ld_relaxed(bar + 1);
   if (threadIdx.x == 0) s_dec_f = -1;
+  if (threadIdx.x < kRowBufs) s_rows[threadIdx.x] = s_merged[threadIdx.x] = 0u;  // ordered by the first table's barriers
   int cb, ce;
   cta_chunk(t0, count, cb, ce);
 
@@ -593,59 +643,31 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
         }
       }
       const int idx = warp_transpose_sum16(v);
-      // Warp rows go to buffer it & 1; warp 0 merges them while the other
-      // warps move on (named barriers: FULL[b] = 1 + b, EMPTY[b] = 3 + b).
-      const int b = it & 1;
-      float (*wr)[17] = s_wrow[b];
-      if (warp != 0 && it >= 2) {  // warp 0 has merged tile it - 2 from this buffer
-        if (b) named_sync<4>();
-        else named_sync<3>();
-      }
+      // The warps' rows of tile `it` go to buffer it % kRowBufs and are merged
+      // by warp it % 8, two tiles later: no warp waits for another unless it
+      // runs kRowBufs tiles ahead, and every warp merges one tile in eight.
+      // (One fixed merging warp, with two buffers and named barriers, kept the
+      // eight warps in step and made that warp the tile's critical path: 256
+      // Huber filters, 5.5M particles, 360.7 -> 352.5 us per step call; 64
+      // learned filters of 100K, 433.9 -> 430.8 us; one filter of 1M particles,
+      // 120.4 -> 119.2 us.)
+      const int b = it % kRowBufs;
+      if (it >= kRowBufs) cta_wait_reach(e, s_merged + b, (unsigned)(it / kRowBufs));  // the buffer is free
       // tiled integer CDF of the systematic resampler, segment level
       const double seg_sum = sys_q ? sys_segment_prefix(e, base, p0, active, lwv, wm, fd->K) : 0.0;
-      if ((lane & 1) == 0 && idx < NV) wr[warp][1 + idx] = v[0];
+      if ((lane & 1) == 0 && idx < NV) s_wrow[b][warp][1 + idx] = v[0];
       if (lane == 0) {
-        wr[warp][0] = wm;
-        s_wq[b][warp] = seg_sum;
+        s_wrow[b][warp][0] = wm;
+        s_wq[b][warp] = sys_q ? seg_sum : -1.0;  // -1: no CDF this step
       }
-      if (warp != 0) {
-        if (b) named_arrive<2>();
-        else named_arrive<1>();
-      } else {
-        if (b) named_sync<2>();
-        else named_sync<1>();
-      }
-      if (warp == 0) {
-        float tm = lane < kWarps ? wr[lane][0] : -INFINITY;
-        tm = warp_max(tm);
-        float acc = 0.f;
-        if (lane < NV && tm > -INFINITY) {
-#pragma unroll
-          for (int w = 0; w < kWarps; ++w) {
-            const float mw = wr[w][0];
-            if (mw > -INFINITY) {
-              float sc = exp2f((mw - tm) * 1.4426950408889634f);
-              if (lane == 1) sc *= sc;
-              acc = fmaf(sc, wr[w][1 + lane], acc);
-            }
-          }
-        }
-        float* row = e.part + (size_t)t * kPartStride;
-        if (lane < NV) row[1 + lane] = acc;
-        if (lane == 0) {
-          row[0] = tm;
-          // filter maximum for the one-pass merge and the integer CDF, kept
-          // only when the filter may resample this epoch
-        }
-        // tile level of the tiled integer CDF
-        if (sys_q) sys_tile_scale(e, t, lane < kWarps ? s_wq[b][lane] : 0.0, lane < kWarps ? wr[lane][0] : -INFINITY, tm);
-        if (it + 2 < ce - cb) {  // buffer b is free again
-          if (b) named_arrive<4>();
-          else named_arrive<3>();
-        }
-      }
+      __syncwarp();
+      if (lane == 0) cta_red_release(s_rows + b);
+      if (it >= kMergeLag && (it - kMergeLag) % kWarps == warp)
+        merge_rows<NV, kWarps>(e, t - kMergeLag, it - kMergeLag, s_wrow, s_wq, s_rows, s_merged);
     }
   }
+  for (int j = max(0, ce - cb - kMergeLag); j < ce - cb; ++j)  // the last tiles
+    if (j % kWarps == warp) merge_rows<NV, kWarps>(e, cb + j, j, s_wrow, s_wq, s_rows, s_merged);
   grid_barrier(e, bar, gen);
 
   // ---------------------------------------------------------------- phase 2
