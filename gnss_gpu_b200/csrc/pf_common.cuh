@@ -104,6 +104,55 @@ __device__ __forceinline__ float2 box_muller_f32(uint32_t a, uint32_t b) {
   return make_float2(r * c, r * s);
 }
 
+// lg2 and rsqrt of the MUFU unit for arguments that are normal numbers (the
+// flush of subnormals spares their range checks).
+__device__ __forceinline__ float lg2_normal(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// box_muller_f32 of M pairs of words (a, b) at once, the same values: every
+// fast logarithm first, then one branch for the words above 1 - 2^-8 among
+// them (a branch per pair would end the block the chains overlap in).  The
+// radicand is positive: -2 log u1 >= 2^-8 on the fast side, >= 2 v > 2^-33 on
+// the other.
+template <int M>
+__device__ __forceinline__ void box_muller_many(const uint32_t (&a)[M], const uint32_t (&b)[M], float (&z0)[M],
+                                                float (&z1)[M]) {
+  const float two_m32 = 2.3283064365386963e-10f;
+  const float half_ulp = 1.1641532182693481e-10f;
+  float l[M];
+  uint32_t top = 0u;
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    l[i] = 0.693147180559945309f * lg2_normal(fmaf((float)a[i], two_m32, half_ulp));
+    top = max(top, a[i]);
+  }
+  if (top >= 0xFF000000u) {
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      const float v = fmaf((float)(~a[i]), two_m32, half_ulp);
+      const float near = -v * fmaf(v, fmaf(v, 1.0f / 3.0f, 0.5f), 1.0f);
+      l[i] = a[i] >= 0xFF000000u ? near : l[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const float q = -2.0f * l[i];
+    const float r = q * rsqrt_normal(q);
+    float s, c;
+    __sincosf(6.283185307179586f * fmaf((float)(b[i] >> 8), 5.9604644775390625e-08f, -0.5f), &s, &c);
+    z0[i] = r * c;
+    z1[i] = r * s;
+  }
+}
+
 __device__ __forceinline__ double2 box_muller_f64(uint32_t a, uint32_t b) {
   const double two_m32 = 2.3283064365386963e-10;
   double u1 = ((double)a + 0.5) * two_m32;

@@ -523,24 +523,7 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
         ds[0] += (float)fe->disp[0];
         ds[1] += (float)fe->disp[1];
         ds[2] += (float)fe->disp[2];
-        const uint32_t fid = (uint32_t)fd->filter_id;
-        const uint32_t k0 = fd->key0, k1 = fd->key1;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          float nz[8];
-          const U4 r = philox10(U4{(uint32_t)(p0 + k), epoch, TAG_PREDICT, fid}, k0, k1);
-          const float2 a = box_muller_f32(r.x, r.y), b = box_muller_f32(r.z, r.w);
-          nz[0] = a.x; nz[1] = a.y; nz[2] = b.x; nz[3] = b.y;
-          if (D > 4) {
-            const U4 r2 = philox10(U4{(uint32_t)(p0 + k), epoch, TAG_PREDICT | 1u, fid}, k0, k1);
-            const float2 c = box_muller_f32(r2.x, r2.y), dd = box_muller_f32(r2.z, r2.w);
-            nz[4] = c.x; nz[5] = c.y; nz[6] = dd.x; nz[7] = dd.y;
-          } else {
-            nz[4] = nz[5] = nz[6] = nz[7] = 0.f;
-          }
-#pragma unroll
-          for (int d = 0; d < D; ++d) x[d][k] = fmaf(fd->sigma[d], nz[d], x[d][k] + ds[d]);
-        }
+        predict4<D>(fd, p0, epoch, ds, x);
       } else {
 #pragma unroll
         for (int d = 0; d < D; ++d)
