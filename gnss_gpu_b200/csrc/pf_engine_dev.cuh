@@ -39,7 +39,7 @@ enum : unsigned {
 // instead of the device faulting.  The release build clamps the same indexes
 // silently (or relies on invariants of the layout) and never sets the bit.
 #ifdef PF_CHECKED
-#define PF_BOUNDS_OK(e, cond) ((cond) ? true : (atomicOr((e).err, ERR_BOUNDS), false))
+#define PF_BOUNDS_OK(e, cond) ((cond) ? true : (raise_err((e), ERR_BOUNDS), false))
 #else
 #define PF_BOUNDS_OK(e, cond) true
 #endif
@@ -128,6 +128,10 @@ struct EngineDev {
   float* sat_dbg;            // mixture mode: per filter and satellite, features and outputs
   unsigned* queue;
   unsigned* err;
+  // pfe_step_io: the host's pinned mirror of the control blocks and of the
+  // error word, which the epoch kernel writes its results to (else null)
+  FilterCtrl* ctrl_map;
+  unsigned* err_map;
   const unsigned char* obs;
   unsigned long long obs_slot_bytes;
   unsigned long long spin_limit;
@@ -145,5 +149,24 @@ struct EngineDev {
   const double* lw64;     // stateless API: FP64 log-weights (else null)
   const double* lw64_max; // device pointer to their maximum
 };
+
+// An epoch's records (pf_filter_epoch_t per filter, then pf_sat_t) as a
+// kernel parameter, when they fit one full satellite table; bytes == 0: they
+// are in EngineDev::obs.
+struct ObsInline {
+  int bytes;
+  int pad_;
+  alignas(8) unsigned char data[sizeof(pf_filter_epoch_t) + PF_MAX_SATS * sizeof(pf_sat_t)];
+};
+static_assert(sizeof(ObsInline) + sizeof(EngineDev) + 64 <= 4096, "kernel parameters");
+
+#ifdef __CUDACC__
+// Sets a bit of the error word, and tells the host's mirror (nonzero is what
+// counts there: the host then reads the word itself).
+__device__ __forceinline__ void raise_err(const EngineDev& e, unsigned bit) {
+  const unsigned old = atomicOr(e.err, bit);
+  if (e.err_map) *(volatile unsigned*)e.err_map = old | bit;
+}
+#endif
 
 }  // namespace pfb

@@ -624,7 +624,7 @@ __device__ __forceinline__ void finalize_filter(const EngineDev& e, const Filter
 #pragma unroll
   for (int d = 0; d < 8; ++d) fc->shift[d] = (recenter && d < D) ? (float)mu[d] : 0.f;
   const bool rs = resample_decision(e, fd, ms, eflags);
-  if ((!(W > 0.0) || !(ms.max_lw > -INFINITY)) && do_weight) atomicOr(e.err, ERR_BAD_WEIGHTS);
+  if ((!(W > 0.0) || !(ms.max_lw > -INFINITY)) && do_weight) raise_err(e, ERR_BAD_WEIGHTS);
   fc->resample_flag = rs ? 1 : 0;
   fc->lw_zero = rs ? 1 : (do_weight ? 0 : (lw_zero ? 1 : 0));
   if (rs) {
@@ -634,6 +634,22 @@ __device__ __forceinline__ void finalize_filter(const EngineDev& e, const Filter
   fc->parity = parity ^ 1;
   fc->epoch = epoch + 1u;
   fc->ticket = 0u;
+  if (e.ctrl_map) {  // results straight into the host's mirror (posted writes)
+    FilterCtrl* h = e.ctrl_map + (fc - e.ctrl);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) h->est_ecef[i] = est[i];
+#pragma unroll
+    for (int c = 0; c < PF_MAX_CLK; ++c) h->est_clk[c] = fc->est_clk[c];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) h->cov[i] = fc->cov[i];
+    h->ess = ess;
+    h->sum_w = W;
+    h->max_lw = ms.max_lw;
+    h->resample_flag = rs ? 1 : 0;
+    h->epoch = epoch + 1u;
+    const unsigned err = *(volatile unsigned*)e.err;  // set by an earlier step
+    if (err) *(volatile unsigned*)e.err_map = err;
+  }
   __threadfence();
 }
 
@@ -691,7 +707,7 @@ __global__ void __launch_bounds__(kThreads, PF_KSTEP_MINB) k_step(EngineDev e, i
     const int eflags = fe->flags;
     int n_sat = fe->n_sat;
     if (n_sat > e.max_sats) {
-      if (threadIdx.x == 0) atomicOr(e.err, ERR_SAT_CAP);
+      if (threadIdx.x == 0) raise_err(e, ERR_SAT_CAP);
       n_sat = e.max_sats;
     }
     if (n_sat < 0) n_sat = 0;
@@ -997,7 +1013,7 @@ __global__ void __launch_bounds__(kThreads) k_scan(EngineDev e, int t0, int coun
           if (spins > 32) __nanosleep(64);
         }
         if (timed_out) {
-          if (threadIdx.x == 0) atomicOr(e.err, ERR_LOOKBACK_TIMEOUT);
+          if (threadIdx.x == 0) raise_err(e, ERR_LOOKBACK_TIMEOUT);
           break;
         }
         __threadfence();
@@ -1086,7 +1102,7 @@ __global__ void __launch_bounds__(kThreads) k_offs(EngineDev e, int t0, int coun
       for (int k = 0; k < 4; ++k) Ck[k] = P + (unsigned long long)sys_inner(E, rho, r, c[k]);
     }
     if (W == 0ull) {  // uniform over the CTA (one filter per tile)
-      if (threadIdx.x == 0) atomicOr(e.err, ERR_BAD_WEIGHTS);
+      if (threadIdx.x == 0) raise_err(e, ERR_BAD_WEIGHTS);
       continue;
     }
     uint32_t Fprev = 0u, Fk[4] = {0u, 0u, 0u, 0u};
@@ -1137,7 +1153,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev& e, const FilterDesc*
   const long long dend = min(d0 + kMergeDiag, 2ll * n);
   const int i0 = (int)__ldcg(e.mp_part + t);
   if (i0 < 0 || i0 >= n) {  // cannot happen with valid weights; never index with it
-    if (threadIdx.x == 0) atomicOr(e.err, ERR_BAD_WEIGHTS);
+    if (threadIdx.x == 0) raise_err(e, ERR_BAD_WEIGHTS);
     return;
   }
   const int win = min(kMergeDiag + 1, n - i0);

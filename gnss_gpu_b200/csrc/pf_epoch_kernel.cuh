@@ -76,7 +76,7 @@ __device__ __forceinline__ void grid_barrier(const EngineDev& e, unsigned* bar, 
     unsigned long long spins = 0;
     while (ld_relaxed(bar + 1) != want) {
       if (++spins > e.spin_limit) {
-        atomicOr(e.err, ERR_BARRIER_TIMEOUT);
+        raise_err(e, ERR_BARRIER_TIMEOUT);
         break;
       }
       if (spins > 64) __nanosleep(32);
@@ -105,7 +105,7 @@ __device__ __forceinline__ void cta_wait_reach(const EngineDev& e, const unsigne
     asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     if ((int)(v - want) >= 0) return;
     if (spins > (1u << 24)) {
-      atomicOr(e.err, ERR_BARRIER_TIMEOUT);
+      raise_err(e, ERR_BARRIER_TIMEOUT);
       return;
     }
   }
@@ -279,7 +279,7 @@ __device__ __forceinline__ void epoch_sys_offspring(const EngineDev& e, int cb, 
       }
       if (threadIdx.x == 0) {
         if (se == tb + nt) fc->wq_total = W;  // the chunk holding the filter's last tile
-        if (W == 0ull) atomicOr(e.err, ERR_BAD_WEIGHTS);
+        if (W == 0ull) raise_err(e, ERR_BAD_WEIGHTS);
       }
       if (W > 0ull) {
         const uint32_t u = ld_cg_u(&fc->sys_u_cur);
@@ -379,7 +379,8 @@ __device__ __forceinline__ void merge_rows(const EngineDev& e, int t, int j, con
 #define PF_EPOCH_MINB 2  // resident CTAs per SM the epoch kernel is compiled for
 #endif
 template <int NCLK, int WMODE, int RESAMPLER>
-__global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, int t0, int count, unsigned* bar) {
+__global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, int t0, int count, unsigned* bar,
+                                                                     const __grid_constant__ ObsInline in) {
   constexpr int D = 3 + NCLK;
   constexpr int NV = 2 + D + 6;
   constexpr int kWarps = kThreads / 32;
@@ -405,6 +406,11 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
   if (threadIdx.x < kRowBufs) s_rows[threadIdx.x] = s_merged[threadIdx.x] = 0u;  // ordered by the first table's barriers
   int cb, ce;
   cta_chunk(t0, count, cb, ce);
+  const unsigned char* const obs0 = in.bytes > 0 ? in.data : e.obs;
+  if (in.bytes > 0 && blockIdx.x == gridDim.x - 1)  // slot 0 keeps them for a later step without an upload
+    for (int i = threadIdx.x * 8; i < in.bytes; i += kThreads * 8)
+      *reinterpret_cast<unsigned long long*>(const_cast<unsigned char*>(e.obs) + i) =
+          *reinterpret_cast<const unsigned long long*>(in.data + i);
 
   // ---------------------------------------------------------------- phase 1
   int cached = -1;
@@ -416,13 +422,13 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
     FilterCtrl* fc = e.ctrl + f;
     const unsigned epoch = fc->epoch;
     const bool lw_zero = fc->lw_zero != 0;
-    const unsigned char* ob = e.obs + (size_t)(epoch % (unsigned)e.obs_slots) * e.obs_slot_bytes;
+    const unsigned char* ob = obs0 + (size_t)(epoch % (unsigned)e.obs_slots) * e.obs_slot_bytes;
     const pf_filter_epoch_t* fe = reinterpret_cast<const pf_filter_epoch_t*>(ob) + f;
     const pf_sat_t* sats = reinterpret_cast<const pf_sat_t*>(ob + sizeof(pf_filter_epoch_t) * e.n_filters);
     const int eflags = fe->flags;
     int n_sat = fe->n_sat;
     if (n_sat > e.max_sats) {
-      if (threadIdx.x == 0) atomicOr(e.err, ERR_SAT_CAP);
+      if (threadIdx.x == 0) raise_err(e, ERR_SAT_CAP);
       n_sat = e.max_sats;
     }
     if (n_sat < 0) n_sat = 0;
@@ -662,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
     const FilterDesc* fd = e.desc + f;
     FilterCtrl* fc = e.ctrl + f;
     const unsigned epoch = fc->epoch;
-    const unsigned char* ob = e.obs + (size_t)(epoch % (unsigned)e.obs_slots) * e.obs_slot_bytes;
+    const unsigned char* ob = obs0 + (size_t)(epoch % (unsigned)e.obs_slots) * e.obs_slot_bytes;
     const pf_filter_epoch_t* fe = reinterpret_cast<const pf_filter_epoch_t*>(ob) + f;
     const int eflags = fe->flags;
     MergedStats ms = merge_tiles<D>(e.part, fd->tile_begin, fd->n_tiles, s_maxtmp, s_dred);
