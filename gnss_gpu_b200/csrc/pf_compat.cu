@@ -112,6 +112,25 @@ int scratch_pool(cudaMemPool_t* out) {
   return PF_OK;
 }
 
+}  // namespace
+
+namespace pfb {
+// `bytes` of stream-ordered scratch (cudaFreeAsync gives it back); null when
+// there is none.
+void* scratch_alloc(size_t bytes, cudaStream_t st) {
+  cudaMemPool_t pool = nullptr;
+  void* p = nullptr;
+  if (pf_injected_alloc_failure() || scratch_pool(&pool) != PF_OK) return nullptr;
+  if (cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+}  // namespace pfb
+
+namespace {
+
 struct Carve {
   unsigned char* base;
   size_t off = 0;

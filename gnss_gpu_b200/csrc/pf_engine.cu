@@ -19,6 +19,10 @@
 
 using namespace pfb;
 
+namespace pfb {
+void* scratch_alloc(size_t bytes, cudaStream_t st);  // pf_compat.cu
+}
+
 struct pf_engine {
   pf_engine_config_t cfg;
   std::vector<pf_filter_params_t> params;
@@ -964,6 +968,56 @@ int pfe_graph_launch(pf_engine_t* eng, int n_epochs) {
 
 namespace {
 
+// The 3D likelihood of one filter: a thread per ray, per particle, or the
+// shadow cells of the cloud (the rule's reasons are at kThreadRays).  The scratch
+// (at most 34 MB) comes from the library's stream-ordered pool and goes back to
+// it within the call; without it every particle's thread walks its own rays.
+int launch_weight_3d(pf_engine_t* eng, int filter, const MeshDev& m, const Sat3d* sv, const Weight3dArgs& a) {
+  const int n = eng->hdesc[filter].n;
+  const int tiles = (n + kThreads - 1) / kThreads;
+  CellBufs cb;
+  memset(&cb, 0, sizeof(cb));
+  unsigned char* buf = nullptr;
+  RayMode mode = RAYS_WALK;
+  if (m.n_nodes > 0 && (long long)n * a.n_sat <= kThreadRays) {
+    const size_t words = (size_t)(n + 31) / 32 * a.n_sat;
+    if ((buf = (unsigned char*)scratch_alloc(sizeof(unsigned) * words, eng->stream))) {
+      mode = RAYS_WORDS;
+      cb.blk = (unsigned*)buf;
+      k_rays_3d<<<(int)std::min<size_t>(eng->sm_count * 16, (words + 7) / 8), kThreads, 0, eng->stream>>>(
+          eng->dev, filter, m, sv, a.n_sat, cb.blk);
+    }
+  } else if (m.n_nodes > 0 && (long long)n * a.n_sat > kCellRays) {
+    const int want = cells_wanted(n, a.n_sat);
+    const size_t blocks = (size_t)(want + want / 4) / kBlockCells + 1, head = 1024 + align_up(blocks / 8 + 4, 256);
+    const size_t codes = align_up(sizeof(unsigned) * blocks * kBlockCells * a.n_sat, 256);
+    static_assert(sizeof(CellGrid) <= 1024, "grid block");
+    buf = (unsigned char*)scratch_alloc(head + codes + sizeof(BlockList) * blocks * a.n_sat, eng->stream);
+    if (buf) {
+      mode = RAYS_CELLS;
+      cb.grid = (CellGrid*)buf;
+      cb.mark = (unsigned*)(buf + 1024);
+      cb.code = (unsigned*)(buf + head);
+      cb.list = (BlockList*)(buf + head + codes);
+      CK(cudaMemsetAsync(buf, 0, head, eng->stream));
+      k_cells_box<<<std::min(eng->sm_count * 2, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, cb.grid,
+                                                                                   a.n_sat);
+      k_cells_mark<<<std::min(eng->sm_count * 4, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, cb);
+      k_cells_block<<<(int)std::min<size_t>(eng->sm_count * 16, (blocks * a.n_sat + 127) / 128), 128, 0,
+                      eng->stream>>>(m, sv, a.n_sat, cb);
+      k_cells_cell<<<(int)std::min<size_t>(eng->sm_count * 8, (blocks * a.n_sat + 7) / 8), kThreads, 0,
+                     eng->stream>>>(m, sv, a.n_sat, cb);
+    }
+  }
+  const auto kernel = mode == RAYS_CELLS   ? k_weight_3d<RAYS_CELLS>
+                      : mode == RAYS_WORDS ? k_weight_3d<RAYS_WORDS>
+                                           : k_weight_3d<RAYS_WALK>;
+  kernel<<<std::min(eng->sm_count * 16, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a, cb);
+  CK(cudaGetLastError());
+  if (buf) CK(cudaFreeAsync(buf, eng->stream));
+  return PF_OK;
+}
+
 void fill_results(pf_engine* eng, pf_filter_result_t* out) {
   for (int f = 0; f < eng->cfg.n_filters; ++f) {
     const FilterCtrl& c = eng->ctrl_host[f];
@@ -1766,14 +1820,7 @@ int pfe_add_3d_term(pf_engine_t* eng, int filter, const pf_mesh_t* mesh, const d
   a.p_clear = p_clear;
   const FilterDesc& d = eng->hdesc[filter];
   const Sat3d* sv = reinterpret_cast<const Sat3d*>(eng->obs_rows);
-  const int g = std::max(1, std::min(eng->sm_count * 16, (d.n + kThreads - 1) / kThreads));
-  switch (eng->D) {
-    case 4: k_weight_3d<4><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a); break;
-    case 5: k_weight_3d<5><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a); break;
-    case 6: k_weight_3d<6><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a); break;
-    default: k_weight_3d<7><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a); break;
-  }
-  CK(cudaGetLastError());
+  if ((s = launch_weight_3d(eng, filter, m, sv, a)) != PF_OK) return s;
   const int zero = 0;
   CK(cudaMemcpyAsync(reinterpret_cast<char*>(eng->ctrl_dev + filter) + offsetof(FilterCtrl, lw_zero), &zero,
                      sizeof(int), cudaMemcpyHostToDevice, eng->stream));
