@@ -1712,13 +1712,9 @@ int pfe_vel_doppler(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const pf_d
   const FilterDesc& d = eng->hdesc[filter];
   double* vb = vs->buf + (size_t)vs->sel * kVelComp * d.n;
   const DopplerRow* dr = reinterpret_cast<const DopplerRow*>(eng->obs_rows);
-  const int g = vel_grid(eng, d.n, 4);
-  switch (eng->D) {
-    case 4: k_doppler<4><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vb, dr, a); break;
-    case 5: k_doppler<5><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vb, dr, a); break;
-    case 6: k_doppler<6><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vb, dr, a); break;
-    default: k_doppler<7><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vb, dr, a); break;
-  }
+  const int g = std::max(1, std::min(eng->sm_count * 16, (d.n + 127) / 128));
+  if (kf) k_doppler<true><<<g, 128, 0, eng->stream>>>(eng->dev, filter, vb, dr, a);
+  else k_doppler<false><<<g, 128, 0, eng->stream>>>(eng->dev, filter, vb, dr, a);
   CK(cudaGetLastError());
   const int zero = 0;
   CK(cudaMemcpyAsync(reinterpret_cast<char*>(eng->ctrl_dev + filter) + offsetof(FilterCtrl, lw_zero), &zero,

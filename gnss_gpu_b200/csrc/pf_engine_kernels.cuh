@@ -436,6 +436,26 @@ __device__ __forceinline__ void load_particles(const EngineDev& e, const FilterD
 }
 
 
+// Where a filter's current particles are (gathered through the last
+// resample, if pending), and the address of particle j's first component.
+struct ParticleSrc {
+  const float* src;
+  const int* seg;
+  long long base;
+  int n;
+  bool gather;
+};
+__device__ __forceinline__ ParticleSrc particle_src(const EngineDev& e, const FilterDesc* fd, const FilterCtrl* fc) {
+  return {fc->parity ? e.state1 : e.state0, seg_markers(e, fd), fd->p_off, fd->n, fc->resample_flag != 0};
+}
+__device__ __forceinline__ const float* particle_at(const EngineDev& e, const ParticleSrc& ps, int j) {
+  if (ps.gather) {
+    const int q = ancestor_at(e, ps.seg, ps.base, j);
+    if ((unsigned)q < (unsigned)ps.n) j = q;
+  }
+  return ps.src + ps.base + j;
+}
+
 // Predict of four particles: x += ds + sigma N(0, 1).  Four normals per
 // Philox block; the blocks of G particles go side by side, in straight-line
 // code, so that their chains (ten Philox rounds, the Box-Muller functions)

@@ -260,25 +260,6 @@ __device__ __forceinline__ void beam_walk(const MeshDev& m, const float3 c, cons
   out->n = kCodePerRay;
 }
 
-// Local offsets of current particle j.
-struct ParticleSrc {
-  const float* src;
-  const int* seg;
-  long long base;
-  int n;
-  bool gather;
-};
-__device__ __forceinline__ ParticleSrc particle_src(const EngineDev& e, const FilterDesc* fd, const FilterCtrl* fc) {
-  return {fc->parity ? e.state1 : e.state0, seg_markers(e, fd), fd->p_off, fd->n, fc->resample_flag != 0};
-}
-__device__ __forceinline__ const float* particle_at(const EngineDev& e, const ParticleSrc& ps, int j) {
-  if (ps.gather) {
-    const int q = ancestor_at(e, ps.seg, ps.base, j);
-    if ((unsigned)q < (unsigned)ps.n) j = q;
-  }
-  return ps.src + ps.base + j;
-}
-
 // Mean and spread of the offsets (exact integer sums, so the grid does not
 // depend on the order), then the grid: cubic cells over the mean +- 4.2
 // standard deviations (outside it rays walk by themselves, 30 times the work),
