@@ -745,9 +745,12 @@ int pf_broadcast_orbits(const pf_broadcast_t* d_recs, int n_recs, const int* d_r
   if (!d_rec_index && n_recs < n_sat) return set_err(PF_EINVAL, "without an index, n_recs must be >= n_sat");
   if (!isfinite(glo_step) || glo_step <= 0.0) glo_step = kGloStep;
   if (glo_step < 1.0) return set_err(PF_EINVAL, "glo_step below 1 s");
-  const long ne = (long)n_epoch * n_sat;
   cudaStream_t st = (cudaStream_t)stream;
-  const unsigned grid = (unsigned)((ne + kB - 1) / kB);
+  const long st_tiles = (n_sat + kTileS - 1) / kTileS, need_tiles = st_tiles * ((n_epoch + 31) / 32);
+  // four epochs per thread once that still gives every SM its CTAs
+  const bool four = need_tiles >= 4 * 148 * 4;
+  const unsigned grid = (unsigned)(st_tiles * ((n_epoch + (four ? 127 : 31)) / (four ? 128 : 32)));
+  const auto orbits = four ? k_broadcast_orbits<4> : k_broadcast_orbits<1>;
   // GLONASS state table: the epochs of a record share its states at whole
   // steps from toe, so they are integrated once per (record, direction)
   int kc = 0;
@@ -757,8 +760,8 @@ int pf_broadcast_orbits(const pf_broadcast_t* d_recs, int n_recs, const int* d_r
     if (kc < 4) kc = 0;  // too many records for the scratch: walk from toe
   }
   if (kc == 0) {
-    k_broadcast_orbits<<<grid, kB, 0, st>>>(d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step,
-                                            nullptr, 0, d_pos, d_clk, nullptr);
+    orbits<<<grid, kTileThreads, 0, st>>>(d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step, nullptr, 0,
+                                          d_pos, d_clk, nullptr);
     CK(cudaGetLastError());
     return PF_OK;
   }
@@ -773,11 +776,25 @@ int pf_broadcast_orbits(const pf_broadcast_t* d_recs, int n_recs, const int* d_r
   double* tbl = (double*)(scratch + kmax_bytes);
   cudaError_t ce = cudaMemsetAsync(kmax, 0, kmax_bytes, st);
   if (ce == cudaSuccess) {
-    k_glo_need<<<grid, kB, 0, st>>>(d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step, kc, kmax);
-    k_glo_table<<<(unsigned)((2 * n_recs + 127) / 128), 128, 0, st>>>(d_recs, n_recs, glo_step, kmax, kc, tbl);
-    k_broadcast_orbits<<<grid, kB, 0, st>>>(d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step, tbl,
-                                            kc, d_pos, d_clk, nullptr);
-    ce = cudaGetLastError();
+    k_glo_need<<<(unsigned)(st_tiles * ((n_epoch + kNeedE - 1) / kNeedE)), kTileThreads, 0, st>>>(
+        d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step, kc, kmax);
+    cudaLaunchConfig_t lc;
+    memset(&lc, 0, sizeof(lc));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    lc.stream = st;
+    lc.gridDim = dim3((unsigned)((2 * n_recs + 31) / 32));  // a serial walk per thread: one warp per CTA
+    lc.blockDim = dim3(32);
+    ce = cudaLaunchKernelEx(&lc, k_glo_table, d_recs, n_recs, glo_step, (const int*)kmax, kc, tbl);
+    if (ce == cudaSuccess) {
+      lc.gridDim = dim3(grid);
+      lc.blockDim = dim3(kTileThreads);
+      ce = cudaLaunchKernelEx(&lc, orbits, d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step,
+                              (const double*)tbl, kc, d_pos, d_clk, (int*)nullptr);
+    }
   }
   const cudaError_t fe = cudaFreeAsync(scratch, st);
   CK(ce);

@@ -81,47 +81,114 @@ __host__ __device__ inline double wrap_half_week(double dt) {
   return dt;
 }
 
-// Kepler's equation by Newton's method from E = M, at most 10 updates,
-// stopping once |dE| < 1e-15 (ephemeris.cu:14-22, ephemeris.py:417-425).
-__device__ inline double kepler_solve(double M, double e) {
-  double E = M;
-  for (int k = 0; k < 10; ++k) {
-    const double dE = (M - E + e * sin(E)) / (1.0 - e * cos(E));
-    E += dE;
-    if (fabs(dE) < 1e-15) break;
+// (s, c) = (sin x, cos x) -> (sin, cos)(x + d) for |d| <= kSmallAngle: the
+// Taylor series of sin d and cos d - 1 (next terms below 1e-24), added to s, c.
+constexpr double kSmallAngle = 0.03;
+__device__ inline void rotate_small(double& s, double& c, double d) {
+  const double d2 = d * d;
+  const double sd = d * (1.0 + d2 * (-1.0 / 6.0 + d2 * (1.0 / 120.0 + d2 * (-1.0 / 5040.0 + d2 / 362880.0))));
+  const double cd = d2 * (-0.5 + d2 * (1.0 / 24.0 + d2 * (-1.0 / 720.0 + d2 / 40320.0)));
+  const double s0 = s;
+  s += s0 * cd + c * sd;
+  c += c * cd - s0 * sd;
+}
+// (sin, cos)(x + d) with x's at hand, for any d.
+__device__ inline void sincos_near(double sx, double cx, double x, double d, double& s, double& c) {
+  if (fabs(d) <= kSmallAngle) {
+    s = sx;
+    c = cx;
+    rotate_small(s, c, d);
+  } else {
+    sincos(x + d, &s, &c);
   }
-  return E;
+}
+
+// 1 / x for x within (1e-30, 1e30): a float reciprocal, refined by Newton's
+// method r += r (1 - x r), N times (each doubles its 24 bits).
+template <int N>
+__device__ inline double recip(double x) {
+  double r = (double)__frcp_rn((float)x);
+#pragma unroll
+  for (int i = 0; i < N; ++i) r = fma(r, fma(-x, r, 1.0), r);
+  return r;
+}
+
+// sin E and cos E of Kepler's equation by Newton's method from E = M, at
+// most 10 updates (ephemeris.cu:14-22, ephemeris.py:417-425).  Sine and cosine
+// follow each update by rotation.  Once an update is below 1e-5 the next
+// one is below 1e-10: sine and cosine are then evaluated at E, and that last
+// update is applied to them (its square is below their rounding).  An update
+// needs no more than the leading digits of its divisor.
+__device__ inline void kepler_solve(double M, double e, double& s, double& c) {
+  double E = M;
+  sincos(M, &s, &c);
+  for (int k = 0; k < 10; ++k) {
+    const double dE = (M - E + e * s) * recip<0>(1.0 - e * c);
+    E += dE;
+    if (fabs(dE) < 1e-5) break;
+    if (fabs(dE) <= kSmallAngle) rotate_small(s, c, dE);
+    else sincos(E, &s, &c);
+  }
+  sincos(E, &s, &c);
+  const double dE = (M - E + e * s) * recip<0>(1.0 - e * c), s0 = s;
+  s += c * dE;
+  c -= s0 * dE;
+}
+
+// What a Kepler record's epochs share.
+struct KeplerShared {
+  double a, n, sq;        // semi-major axis, mean motion, sqrt(1 - e^2)
+  double so, co, si, ci;  // of the argument of perigee and of i0
+  double om_rate, om_toe, rel;
+};
+__device__ inline KeplerShared kepler_shared(const pf_ephemeris_t& k, int system) {
+  const OrbitConsts c = orbit_consts(system);
+  KeplerShared o;
+  o.a = k.sqrt_a * k.sqrt_a;
+  o.n = sqrt(c.mu / (o.a * o.a * o.a)) + k.delta_n;
+  o.sq = sqrt(1.0 - k.e * k.e);
+  sincos(k.omega, &o.so, &o.co);
+  sincos(k.i0, &o.si, &o.ci);
+  o.om_rate = k.omega_dot - c.omega_e;
+  o.om_toe = c.omega_e * k.toe;
+  o.rel = c.rel_f * k.e * k.sqrt_a;
+  return o;
 }
 
 // Position (ECEF, m) and clock correction (s) of a Kepler record at GPST
 // second of week t (ephemeris.py:428-512; the GPS-only kernel of
 // ephemeris.cu:24-104 is system 'G').  The record's tgd is subtracted as
 // stored; callers put the group delay they want there (0 to omit it).
-__device__ inline void kepler_orbit(const pf_ephemeris_t& k, int system, double t, double* pos,
+//
+// The angles: sine and cosine of the true anomaly are algebraic in those of
+// E, the argument of latitude and the inclination are small corrections of
+// angles whose sine and cosine are known, so three sincos per epoch (M, E, the
+// node) take the place of an arc tangent and some fifteen sines and cosines.
+__device__ inline void kepler_orbit(const pf_ephemeris_t& k, const KeplerShared& o, int system, double t, double* pos,
                                     double* clk) {
-  const OrbitConsts c = orbit_consts(system);
-  const double a = k.sqrt_a * k.sqrt_a;
-  const double n = sqrt(c.mu / (a * a * a)) + k.delta_n;
   const double rx = broadcast_rx_sow(system, t);
   const double tk = wrap_half_week(rx - k.toe);
-  const double E = kepler_solve(k.M0 + n * tk, k.e);
-  const double sE = sin(E), cE = cos(E);
-  const double den = 1.0 - k.e * cE;
-  const double v = atan2(sqrt(1.0 - k.e * k.e) * sE / den, (cE - k.e) / den);
-  const double phi = v + k.omega;
-  const double s2 = sin(2.0 * phi), c2 = cos(2.0 * phi);
-  const double u = phi + (k.cuc * c2 + k.cus * s2);
-  const double r = a * (1.0 - k.e * cE) + (k.crc * c2 + k.crs * s2);
-  const double inc = k.i0 + k.idot * tk + (k.cic * c2 + k.cis * s2);
-  const double xp = r * cos(u), yp = r * sin(u);
-  const double Om = k.omega0 + (k.omega_dot - c.omega_e) * tk - c.omega_e * k.toe;
-  const double cO = cos(Om), sO = sin(Om), ci = cos(inc), si = sin(inc);
+  double sE, cE;
+  kepler_solve(k.M0 + o.n * tk, k.e, sE, cE);
+  const double den = 1.0 - k.e * cE, iden = recip<2>(den);
+  const double sv = o.sq * sE * iden, cv = (cE - k.e) * iden;
+  const double sp = sv * o.co + cv * o.so, cp = cv * o.co - sv * o.so;  // phi = v + omega
+  const double s2 = 2.0 * sp * cp, c2 = cp * cp - sp * sp;
+  const double du = k.cuc * c2 + k.cus * s2;
+  double su = sp, cu = cp;
+  if (fabs(du) <= kSmallAngle) rotate_small(su, cu, du);
+  else sincos(atan2(sp, cp) + du, &su, &cu);
+  const double r = o.a * den + (k.crc * c2 + k.crs * s2);
+  double si, ci;
+  sincos_near(o.si, o.ci, k.i0, k.idot * tk + (k.cic * c2 + k.cis * s2), si, ci);
+  const double xp = r * cu, yp = r * su;
+  double sO, cO;
+  sincos(k.omega0 + o.om_rate * tk - o.om_toe, &sO, &cO);
   pos[0] = xp * cO - yp * ci * sO;
   pos[1] = xp * sO + yp * ci * cO;
   pos[2] = yp * si;
   const double dt = wrap_half_week(rx - k.toc);
-  const double dtr = c.rel_f * k.e * k.sqrt_a * sE;
-  *clk = k.af0 + k.af1 * dt + k.af2 * dt * dt + dtr - k.tgd;
+  *clk = k.af0 + k.af1 * dt + k.af2 * dt * dt + o.rel * sE - k.tgd;
 }
 
 // PZ-90 equations of motion with the broadcast luni-solar acceleration
@@ -132,11 +199,11 @@ __device__ inline void glo_deriv(const double* x, const double* acc, double* d) 
     for (int i = 0; i < 6; ++i) d[i] = 0.0;
     return;
   }
-  const double r3 = r2 * sqrt(r2);
+  const double ir = rsqrt(r2), ir2 = ir * ir, ir3 = ir2 * ir;  // one reciprocal root, no division
   const double w2 = kGloOmega * kGloOmega;
-  const double at = 1.5 * kGloJ2 * kGloMu * (kGloRe * kGloRe) / r2 / r3;
-  const double bt = 5.0 * x[2] * x[2] / r2;
-  const double ct = -kGloMu / r3 - at * (1.0 - bt);
+  const double at = 1.5 * kGloJ2 * kGloMu * (kGloRe * kGloRe) * ir2 * ir3;
+  const double bt = 5.0 * x[2] * x[2] * ir2;
+  const double ct = -kGloMu * ir3 - at * (1.0 - bt);
   d[0] = x[3];
   d[1] = x[4];
   d[2] = x[5];
@@ -162,12 +229,30 @@ __device__ inline void glo_rk4(double h, double* x, const double* acc) {
 // week t and what is left for the residual step: the loop of
 // orbit_glonass.py:122-150 without the arithmetic (rem decremented in the
 // same order, so it is bit-identical).  Returns false past kGloMaxSteps.
+//
+// With a whole number of seconds per step every difference is exact (it lies
+// on the grid of el's last bit), so the count is a quotient.
 __device__ inline bool glo_plan(const pf_glonass_state_t& g, double t, double step, double& el, double& base,
                                 long& k, double& rem) {
   el = wrap_half_week(broadcast_rx_sow('R', t) - g.toe);
   base = el < 0.0 ? -step : step;
   rem = el;
   k = 0;
+  if (step == rint(step) && fabs(el) < 1e9) {  // |el| <= half a week unless the input is wild
+    double q = floor(fabs(el) / step);
+    double left = fma(-q, step, fabs(el));
+    if (left < 0.0) {  // the quotient was rounded up
+      q -= 1.0;
+      left += step;
+    } else if (left >= step) {
+      q += 1.0;
+      left -= step;
+    }
+    if (q > (double)kGloMaxSteps) return false;
+    k = (long)q;
+    rem = el < 0.0 ? -left : left;
+    return true;
+  }
   // a NaN time takes no step (the reference returns the broadcast position
   // with a NaN clock); an infinite one runs into the step bound
   while (fabs(rem) >= fabs(base)) {  // |base| >= 1 s, so |rem| > 1e-9 here
@@ -215,38 +300,66 @@ __device__ inline int orbit_record(const int* idx, long i, int s, int n_recs) {
   return (r < 0 || r >= n_recs) ? -1 : r;
 }
 
+// Tiles of kTileE epochs x 8 satellites per CTA: a warp takes epochs of one
+// satellite, so its lanes run the same orbit model with similar step counts, and
+// the CTA's eight satellites make the row-major arrays' segments (8 indexes, 8
+// positions, 8 clocks of an epoch) whole sectors.
+constexpr int kTileS = 8;
+constexpr int kTileThreads = 32 * kTileS;
+
+// Programmatic dependent launch: the state table is needed by GLONASS tiles
+// only, so the orbit kernel starts while the table is made.
+__device__ inline void orbit_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ inline void orbit_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Deepest stored state each (GLONASS record, direction) needs: kmax[2r + d]
-// = max over its satellite-epochs of min(full steps, kc).
-__global__ void k_glo_need(const pf_broadcast_t* __restrict__ recs, int n_recs, const int* __restrict__ idx,
-                           const double* __restrict__ times, int n_epoch, int n_sat, double step, int kc,
-                           int* __restrict__ kmax) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+// >= max over its satellite-epochs of min(full steps, kc).  Whole steps of the
+// walk (glo_plan) are at most |el| / step rounded up.  A lane follows its
+// satellite through kNeedE / 32 epochs and raises the count of a record when it
+// leaves it (an atomic per satellite-epoch took 150 us on a day of 24 satellites).
+constexpr int kNeedE = 512;
+__global__ void __launch_bounds__(kTileThreads) k_glo_need(const pf_broadcast_t* __restrict__ recs, int n_recs,
+                           const int* __restrict__ idx, const double* __restrict__ times, int n_epoch, int n_sat,
+                           double step, int kc, int* __restrict__ kmax) {
+  orbit_pdl_trigger();
+  const int st = (n_sat + kTileS - 1) / kTileS;
+  const int s = (int)(blockIdx.x % st) * kTileS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (s >= n_sat) return;  // whole warps
+  const int e0 = (int)(blockIdx.x / st) * kNeedE, e1 = min(n_epoch, e0 + kNeedE);
   int slot = -1, need = 0;
-  if (t < (long)n_epoch * n_sat) {
-    const int s = (int)(t / n_epoch), e = (int)(t - (long)s * n_epoch);
+  auto raise = [&](int sl, int m) {
+    if (*(volatile int*)(kmax + sl) < m) atomicMax(kmax + sl, m);
+  };
+  for (int e = e0 + lane; e < e1; e += 32) {
     const int r = orbit_record(idx, (long)e * n_sat + s, s, n_recs);
-    double el, base, rem;
-    long k;
-    if (r >= 0 && recs[r].system == 'R' && glo_plan(recs[r].u.glonass, times[e], step, el, base, k, rem) && k > 0) {
-      slot = 2 * r + (base < 0.0 ? 1 : 0);
-      need = (int)(k < kc ? k : kc);
+    if (r < 0 || recs[r].system != 'R') continue;
+    const double el = wrap_half_week(broadcast_rx_sow('R', times[e]) - recs[r].u.glonass.toe);
+    const double k = ceil(fabs(el) / step);
+    if (!(k >= 1.0)) continue;  // also NaN
+    const int sl = 2 * r + (el < 0.0 ? 1 : 0);
+    if (sl != slot) {
+      if (slot >= 0) raise(slot, need);
+      slot = sl;
+      need = 0;
     }
+    need = max(need, k < (double)kc ? (int)k : kc);
   }
-  // satellite-major order: a warp's lanes are consecutive epochs of one
-  // satellite and mostly share a slot, so one atomic per group of lanes
+  __syncwarp();
   const unsigned grp = __match_any_sync(0xffffffffu, slot);
   const int m = (int)__reduce_max_sync(grp, (unsigned)need);
-  if (slot >= 0 && (threadIdx.x & 31) == __ffs(grp) - 1) atomicMax(kmax + slot, m);
+  if (slot >= 0 && lane == __ffs(grp) - 1) raise(slot, m);
 }
 
 // The stored states: one thread per (record, direction) integrates kmax
 // full steps from toe and keeps every state (6 doubles each, kc per slot).
 __global__ void k_glo_table(const pf_broadcast_t* __restrict__ recs, int n_recs, double step,
                             const int* __restrict__ kmax, int kc, double* __restrict__ tbl) {
+  orbit_pdl_trigger();
+  orbit_pdl_wait();  // kmax
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 2 * n_recs) return;
-  const int K = kmax[t];
-  if (K <= 0) return;
+  const int K = __ldcg(kmax + t);
+  if (K <= 0 || recs[t >> 1].system != 'R') return;
   const pf_glonass_state_t& g = recs[t >> 1].u.glonass;
   const double h = (t & 1) ? -step : step;
   double x[6] = {g.pos[0], g.pos[1], g.pos[2], g.vel[0], g.vel[1], g.vel[2]};
@@ -261,39 +374,78 @@ __global__ void k_glo_table(const pf_broadcast_t* __restrict__ recs, int n_recs,
 // is null) at times[e]; an index outside [0, n_recs) gives NaN, and so does a
 // GLONASS integration past kGloMaxSteps steps (also flagged in *err if given).
 // tbl / kc: the GLONASS state table of k_glo_table, or null / 0.
-// Three CTAs of 256 per SM (80 registers): the walk is FP64-latency bound,
-// and the extra warps hide more of it than the few spilled values cost.
-__global__ void __launch_bounds__(256, 3) k_broadcast_orbits(const pf_broadcast_t* __restrict__ recs, int n_recs,
+//
+// FP64 bound (36 bytes a satellite-epoch are 31 us of the day-long call at
+// the measured copy rate).  Each thread takes EPT epochs of its satellite and
+// keeps what its record's epochs share; results go through shared memory, so
+// that positions and clocks leave as whole rows of eight satellites.  A day at
+// 1 Hz of 40 Kepler and 24 GLONASS satellites, the whole call: 495 -> 247 us.
+// Four CTAs per SM (64 registers): with two 291 us, with three 258.
+template <int EPT>
+__global__ void __launch_bounds__(kTileThreads, 4) k_broadcast_orbits(const pf_broadcast_t* __restrict__ recs, int n_recs,
                                    const int* __restrict__ idx, const double* __restrict__ times,
                                    int n_epoch, int n_sat, double glo_step, const double* __restrict__ tbl, int kc,
                                    double* __restrict__ pos, double* __restrict__ clk, int* __restrict__ err) {
-  // Satellite-major thread order: a warp covers 32 consecutive epochs of one
-  // satellite, so its lanes run the same orbit model (Kepler or the longer
-  // GLONASS integration) with similar step counts.
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long)n_epoch * n_sat) return;
-  const int s = (int)(t / n_epoch), e = (int)(t - (long)s * n_epoch);
-  const long i = (long)e * n_sat + s;
-  const int r = orbit_record(idx, i, s, n_recs);
-  double p[3], c;
-  if (r < 0) {
+  constexpr int kE = 32 * EPT;
+  __shared__ int s_idx[kE][kTileS + 1];
+  __shared__ double s_pos[32][3 * kTileS + 1];
+  __shared__ double s_clk[32][kTileS + 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int st = (n_sat + kTileS - 1) / kTileS, et = (n_epoch + kE - 1) / kE;
+  // satellites slowest: GLONASS satellites, mostly at the end of the list,
+  // come last and find their table ready
+  const int s0 = (int)(blockIdx.x / et) * kTileS, e0 = (int)(blockIdx.x % et) * kE;
+  const int ns = min(kTileS, n_sat - s0);
+  if (s0 >= st * kTileS) return;
+  for (int i = threadIdx.x; i < kE * kTileS; i += kTileThreads) {
+    const int e = e0 + i / kTileS, s = s0 + i % kTileS;
+    s_idx[i / kTileS][i % kTileS] = e < n_epoch && s < n_sat ? orbit_record(idx, (long)e * n_sat + s, s, n_recs) : -1;
+  }
+  __syncthreads();
+  KeplerShared sh;
+  int have = -1;
+  bool waited = false;
+#pragma unroll 1
+  for (int q = 0; q < EPT && e0 + 32 * q < n_epoch; ++q) {
+    const int e = e0 + 32 * q + lane, r = s_idx[32 * q + lane][w];
+    double p[3], c;
     p[0] = p[1] = p[2] = c = nan("");
-  } else {
-    const pf_broadcast_t& rec = recs[r];
-    if (rec.system == 'R') {
-      const double el = wrap_half_week(broadcast_rx_sow('R', times[e]) - rec.u.glonass.toe);
-      const double* tb = tbl ? tbl + ((size_t)2 * r + (el < 0.0 ? 1 : 0)) * kc * 6 : nullptr;
-      if (!glonass_orbit(rec.u.glonass, times[e], glo_step, tb, kc, p, &c) && err) atomicOr(err, 1);
-    } else {
-      kepler_orbit(rec.u.kepler, rec.system, times[e], p, &c);
+    const bool glo = r >= 0 && recs[r].system == 'R';
+    if (tbl && !waited && __any_sync(0xffffffffu, glo)) {
+      orbit_pdl_wait();
+      waited = true;
     }
+    if (glo) {
+      const pf_glonass_state_t& g = recs[r].u.glonass;
+      const double el = wrap_half_week(broadcast_rx_sow('R', times[e]) - g.toe);
+      const double* tb = tbl ? tbl + ((size_t)2 * r + (el < 0.0 ? 1 : 0)) * kc * 6 : nullptr;
+      if (!glonass_orbit(g, times[e], glo_step, tb, kc, p, &c) && err) atomicOr(err, 1);
+    } else if (r >= 0) {
+      const pf_ephemeris_t& k = recs[r].u.kepler;
+      if (r != have) {
+        sh = kepler_shared(k, recs[r].system);
+        have = r;
+      }
+      kepler_orbit(k, sh, recs[r].system, times[e], p, &c);
+    }
+    __syncthreads();  // the previous rows have left
+    s_pos[lane][3 * w] = p[0];
+    s_pos[lane][3 * w + 1] = p[1];
+    s_pos[lane][3 * w + 2] = p[2];
+    s_clk[lane][w] = c;
+    __syncthreads();
+    const int rows = min(32, n_epoch - (e0 + 32 * q));
+    const long row0 = (long)(e0 + 32 * q) * n_sat + s0;
+    if (pos)
+      for (int i = threadIdx.x; i < rows * 3 * kTileS; i += kTileThreads) {
+        const int er = i / (3 * kTileS), k = i % (3 * kTileS);
+        if (k < 3 * ns) pos[3 * (row0 + (long)er * n_sat) + k] = s_pos[er][k];
+      }
+    if (clk)
+      for (int i = threadIdx.x; i < rows * kTileS; i += kTileThreads)
+        if (i % kTileS < ns) clk[row0 + (long)(i / kTileS) * n_sat + i % kTileS] = s_clk[i / kTileS][i % kTileS];
   }
-  if (pos) {
-    pos[3 * i] = p[0];
-    pos[3 * i + 1] = p[1];
-    pos[3 * i + 2] = p[2];
-  }
-  if (clk) clk[i] = c;
+  if (tbl && !waited) orbit_pdl_wait();  // the grid ends after the table's
 }
 
 // GPS-constant batch over the reference's parameter array
@@ -304,7 +456,7 @@ __global__ void k_sat_pos_gps(const pf_ephemeris_t* __restrict__ params, const d
   if (i >= (long)n_epoch * n_sat) return;
   const int e = (int)(i / n_sat), s = (int)(i - (long)e * n_sat);
   double p[3], c;
-  kepler_orbit(params[s], 'G', times[e], p, &c);
+  kepler_orbit(params[s], kepler_shared(params[s], 'G'), 'G', times[e], p, &c);
   pos[3 * i] = p[0];
   pos[3 * i + 1] = p[1];
   pos[3 * i + 2] = p[2];
