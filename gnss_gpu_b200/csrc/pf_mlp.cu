@@ -6,14 +6,21 @@
 //   L = BCE(sigmoid(o0), nlos) + nlos * ((mu - b) / 20 m)^2,  mu = 20 m softplus(o1)
 // averaged over the batch.
 //
-// k_mlp_grad: each CTA takes rounds of 128 rows (8 warps x 16); per round a
+// k_mlp_grad: each CTA takes rounds of 64 rows (4 warps x 16); per round a
 // warp runs the forward pass and the backward pass of its rows on the tensor
 // cores (dO -> dH2 = dO W3 masked by ReLU' -> dH1 = dH2 W2^T masked), stages
 // activations and gradients in shared memory as BF16, and the CTA then forms
-// the weight gradients dW = G^T H over the round's 128 rows, again as MMAs,
-// accumulated across rounds in registers.  Per-CTA partial gradients go to a
-// scratch array and k_mlp_reduce sums them in a fixed order (deterministic),
-// then applies Adam or returns the gradient.
+// the weight gradients dW = G^T H over the round's rows, again as MMAs (the bias
+// gradients as products with ones), accumulated across rounds in registers.
+// Per-CTA partial gradients go to a scratch array and k_mlp_reduce sums them in
+// a fixed order (deterministic), then applies Adam or returns the gradient.
+//
+// A step on the default batch (8192 rows) is a latency chain: load, three
+// layers forward, three back, weight gradients, reduction.  64 rows per CTA put
+// it on 128 of 148 SMs (128 rows: on 64), transposed operands come by ldmatrix
+// from padded rows (scalar two-byte loads before), and the two kernels of a step
+// start while their predecessor drains.  Step of 8192 rows 32.8 -> 12.6 us, of
+// 100,000 rows 239 -> 35 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -25,82 +32,98 @@
 
 namespace pfb {
 
-constexpr int kMlpThreads = 256;
-constexpr int kRows = 128;  // rows per CTA round
+constexpr int kMlpThreads = 128;
+constexpr int kRows = 64;  // rows per CTA round
+constexpr int kLdH = mlp_ld(kMlpH), kLdX = mlp_ld(kMlpIn);
+constexpr int kMlpPart = kMlpParams + 1;  // floats per partial gradient (and its loss)
 
 struct GradSmem {
   MlpSmem w;
-  float x[kRows * kMlpIn];          // inputs, FP32, cols 12..15 zero
-  __nv_bfloat16 h1[kRows * kMlpH];  // activations after ReLU
-  __nv_bfloat16 h2[kRows * kMlpH];
-  __nv_bfloat16 g1[kRows * kMlpH];  // dL/d(pre-activation) of layer 1
-  __nv_bfloat16 g2[kRows * kMlpH];  // of layer 2
-  __nv_bfloat16 go[kRows * 16];     // dL/do (cols 0, 1), zero padded
+  float x[kRows * kMlpIn];                     // inputs, FP32, cols 12..15 zero
+  alignas(16) __nv_bfloat16 xb[kRows * kLdX];  // the same in BF16
+  alignas(16) __nv_bfloat16 h1[kRows * kLdH];  // activations after ReLU
+  alignas(16) __nv_bfloat16 h2[kRows * kLdH];
+  alignas(16) __nv_bfloat16 g1[kRows * kLdH];  // dL/d(pre-activation) of layer 1
+  alignas(16) __nv_bfloat16 g2[kRows * kLdH];  // of layer 2
+  alignas(16) __nv_bfloat16 go[kRows * kLdX];  // dL/do (cols 0, 1), zero padded
   float loss[kMlpThreads / 32];
 };
+
+__device__ __forceinline__ void mlp_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void mlp_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Store a BF16 A fragment (k-tile q) of rows [r0, r0+16) into a row-major
 // [rows][64] BF16 array.
 __device__ __forceinline__ void store_frag(__nv_bfloat16* dst, int r0, int q, int lane, const uint32_t (&a)[4]) {
   const int g = lane >> 2, t = lane & 3;
-  *reinterpret_cast<uint32_t*>(dst + (size_t)(r0 + g) * kMlpH + 16 * q + 2 * t) = a[0];
-  *reinterpret_cast<uint32_t*>(dst + (size_t)(r0 + g + 8) * kMlpH + 16 * q + 2 * t) = a[1];
-  *reinterpret_cast<uint32_t*>(dst + (size_t)(r0 + g) * kMlpH + 16 * q + 8 + 2 * t) = a[2];
-  *reinterpret_cast<uint32_t*>(dst + (size_t)(r0 + g + 8) * kMlpH + 16 * q + 8 + 2 * t) = a[3];
+  *reinterpret_cast<uint32_t*>(dst + (r0 + g) * kLdH + 16 * q + 2 * t) = a[0];
+  *reinterpret_cast<uint32_t*>(dst + (r0 + g + 8) * kLdH + 16 * q + 2 * t) = a[1];
+  *reinterpret_cast<uint32_t*>(dst + (r0 + g) * kLdH + 16 * q + 8 + 2 * t) = a[2];
+  *reinterpret_cast<uint32_t*>(dst + (r0 + g + 8) * kLdH + 16 * q + 8 + 2 * t) = a[3];
 }
 
-__device__ __forceinline__ uint32_t pack_raw(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-  return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
-}
 __device__ __forceinline__ float bf(uint32_t v, int hi) {
   return __bfloat162float(__ushort_as_bfloat16((unsigned short)(hi ? (v >> 16) : (v & 0xFFFFu))));
 }
 
-// A fragment of the transposed operand: A[m][k] = src[k][m] for the tile of
-// rows m in [16 mt, 16 mt + 16) and k in [16 kt, 16 kt + 16); src is
-// [kRows][ld] BF16 (zero where m >= valid_m).
+// Four 8x8 blocks of a row-major BF16 matrix, transposed: block j's rows start
+// at the addresses of lanes 8j..8j+7.
+__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p))
+               : "memory");
+}
+// A fragment of the transposed operand: A[m][k] = src[k][m] for m in [16 mt,
+// 16 mt + 16), k in [16 kt, 16 kt + 16); src is row-major with stride LD.
 template <int LD>
 __device__ __forceinline__ void a_frag_t(const __nv_bfloat16* src, int mt, int kt, int lane, uint32_t (&a)[4]) {
-  const int g = lane >> 2, t = lane & 3;
-  const int m0 = 16 * mt + g, k0 = 16 * kt + 2 * t;
-  a[0] = pack_raw(src[(size_t)k0 * LD + m0], src[(size_t)(k0 + 1) * LD + m0]);
-  a[1] = pack_raw(src[(size_t)k0 * LD + m0 + 8], src[(size_t)(k0 + 1) * LD + m0 + 8]);
-  a[2] = pack_raw(src[(size_t)(k0 + 8) * LD + m0], src[(size_t)(k0 + 9) * LD + m0]);
-  a[3] = pack_raw(src[(size_t)(k0 + 8) * LD + m0 + 8], src[(size_t)(k0 + 9) * LD + m0 + 8]);
+  const int j = lane >> 3, r = lane & 7;  // blocks: (k, m), (k, m + 8), (k + 8, m), (k + 8, m + 8)
+  ldsm_x4_t(a, src + (16 * kt + (j >> 1) * 8 + r) * LD + 16 * mt + (j & 1) * 8);
 }
-// B fragment B[k][n] = src[k][n], src [kRows][LD] BF16.
+// B fragments of n-tiles nt, nt + 1: B[k][n] = src[k][n], (b[0], b[1]) and (b[2], b[3]).
 template <int LD>
-__device__ __forceinline__ void b_frag_rows(const __nv_bfloat16* src, int kt, int nt, int lane, uint32_t& b0, uint32_t& b1) {
-  const int g = lane >> 2, t = lane & 3;
-  const int n = 8 * nt + g, k0 = 16 * kt + 2 * t;
-  b0 = pack_raw(src[(size_t)k0 * LD + n], src[(size_t)(k0 + 1) * LD + n]);
-  b1 = pack_raw(src[(size_t)(k0 + 8) * LD + n], src[(size_t)(k0 + 9) * LD + n]);
+__device__ __forceinline__ void b_frag_rows2(const __nv_bfloat16* src, int kt, int nt, int lane, uint32_t (&b)[4]) {
+  const int j = lane >> 3, r = lane & 7;  // blocks: (k, n), (k + 8, n), (k, n + 8), (k + 8, n + 8)
+  ldsm_x4_t(b, src + (16 * kt + (j & 1) * 8 + r) * LD + 8 * nt + (j >> 1) * 8);
 }
 
-__global__ void __launch_bounds__(kMlpThreads, 1)
+__global__ void __launch_bounds__(kMlpThreads, 2)
     k_mlp_grad(const float* __restrict__ X, const float* __restrict__ Y, int n, const float* __restrict__ prm,
                float inv_n, float* __restrict__ partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  mlp_pdl_trigger();
+  mlp_pdl_wait();
   mlp_stage(prm, S.w, kMlpThreads);
 
-  float acc2[4][4], acc1[4], acc3[4];  // dW2t (4 m-tiles of n-tile warp), dW1t block, dW3t n-tile warp
+  // warp w: dW2t n-tiles 2w, 2w + 1 (all four m-tiles), dW1t m-tile w (both
+  // n-tiles), dW3t n-tiles 2w, 2w + 1, bias gradients of m-tile w (db1, db2; warp 0 db3)
+  float acc2[4][2][4], acc1[2][4], acc3[2][4], ab1[4], ab2[4], ab3[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    acc1[i] = 0.f;
-    acc3[i] = 0.f;
+    ab1[i] = ab2[i] = ab3[i] = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc2[i][j] = 0.f;
+    for (int h = 0; h < 2; ++h) {
+      acc1[h][i] = acc3[h][i] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc2[j][h][i] = 0.f;
+    }
   }
-  float bacc = 0.f;  // bias gradient owned by this thread (b1: 0..63, b2: 64..127, b3: 128..129)
+  const uint32_t ones = 0x3F803F80u;  // two BF16 ones
   float lsum = 0.f;
 
   for (int base = blockIdx.x * kRows; base < n; base += gridDim.x * kRows) {
     __syncthreads();  // previous round's shared data consumed; weights staged
-    for (int i = threadIdx.x; i < kRows * kMlpIn; i += kMlpThreads) {
-      const int r = i / kMlpIn, c = i % kMlpIn;
-      S.x[i] = (base + r < n && c < kMlpFeat) ? X[(size_t)(base + r) * kMlpFeat + c] : 0.f;
+    for (int i = threadIdx.x; i < kRows * kMlpIn / 2; i += kMlpThreads) {
+      const int r = i / (kMlpIn / 2), c = 2 * (i % (kMlpIn / 2));
+      const bool in = base + r < n && c < kMlpFeat;
+      const float x0 = in ? X[(size_t)(base + r) * kMlpFeat + c] : 0.f;
+      const float x1 = in ? X[(size_t)(base + r) * kMlpFeat + c + 1] : 0.f;
+      S.x[r * kMlpIn + c] = x0;
+      S.x[r * kMlpIn + c + 1] = x1;
+      *reinterpret_cast<uint32_t*>(S.xb + r * kLdX + c) = pack_bf16(x0, x1);
     }
     __syncthreads();
     const int r0 = warp * 16;
@@ -134,25 +157,31 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
     ad[3] = 0u;
     if (t != 0) ad[0] = ad[1] = 0u;
     {
-      uint32_t* gr = reinterpret_cast<uint32_t*>(S.go + (size_t)(r0 + g) * 16 + 2 * t);
-      uint32_t* gr8 = reinterpret_cast<uint32_t*>(S.go + (size_t)(r0 + g + 8) * 16 + 2 * t);
+      uint32_t* gr = reinterpret_cast<uint32_t*>(S.go + (r0 + g) * kLdX + 2 * t);
+      uint32_t* gr8 = reinterpret_cast<uint32_t*>(S.go + (r0 + g + 8) * kLdX + 2 * t);
       gr[0] = ad[0];
       gr8[0] = ad[1];
-      *reinterpret_cast<uint32_t*>(S.go + (size_t)(r0 + g) * 16 + 8 + 2 * t) = 0u;
-      *reinterpret_cast<uint32_t*>(S.go + (size_t)(r0 + g + 8) * 16 + 8 + 2 * t) = 0u;
+      gr[4] = 0u;
+      gr8[4] = 0u;
     }
     // dH2 = dO W3 (B[k = out][n = hidden] = W3t[out][hidden], zero for out >= 2), masked by ReLU'(H2)
     uint32_t gh2[4][4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       float c[2][4];
+      uint32_t b[2];  // k 0..7 of n-tiles 2q, 2q + 1 (rows 2..7 are zero; k 8..15 likewise)
+      {
+        const __nv_bfloat16* p = S.w.w3t + (lane & 7) * kLdH + 16 * q + ((lane >> 3) & 1) * 8;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+                     : "=r"(b[0]), "=r"(b[1])
+                     : "r"((uint32_t)__cvta_generic_to_shared(p))
+                     : "memory");
+      }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int nn = 8 * (2 * q + h) + g;
-        const uint32_t b0 = (t == 0) ? pack_raw(S.w.w3t[nn], S.w.w3t[kMlpH + nn]) : 0u;
 #pragma unroll
         for (int i = 0; i < 4; ++i) c[h][i] = 0.f;
-        mma_bf16(c[h], ad, b0, 0u);
+        mma_bf16(c[h], ad, b[h], 0u);
       }
       // mask: the same lane holds H2 at the same (row, col) in fragment q
       gh2[q][0] = pack_bf16(bf(T.h2[q][0], 0) > 0.f ? c[0][0] : 0.f, bf(T.h2[q][0], 1) > 0.f ? c[0][1] : 0.f);
@@ -165,17 +194,15 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
     for (int q = 0; q < 4; ++q) {
       float c[2][4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int nn = 8 * (2 * q + h) + g;
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int i = 0; i < 4; ++i) c[h][i] = 0.f;
 #pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-          const int k0 = 16 * kt + 2 * t;
-          const uint32_t b0 = pack_raw(S.w.w2t[(size_t)k0 * kMlpH + nn], S.w.w2t[(size_t)(k0 + 1) * kMlpH + nn]);
-          const uint32_t b1 = pack_raw(S.w.w2t[(size_t)(k0 + 8) * kMlpH + nn], S.w.w2t[(size_t)(k0 + 9) * kMlpH + nn]);
-          mma_bf16(c[h], gh2[kt], b0, b1);
-        }
+      for (int kt = 0; kt < 4; ++kt) {
+        uint32_t b[4];
+        b_frag_rows2<kLdH>(S.w.w2t, kt, 2 * q, lane, b);
+        mma_bf16(c[0], gh2[kt], b[0], b[1]);
+        mma_bf16(c[1], gh2[kt], b[2], b[3]);
       }
       uint32_t gq[4];
       gq[0] = pack_bf16(bf(T.h1[q][0], 0) > 0.f ? c[0][0] : 0.f, bf(T.h1[q][0], 1) > 0.f ? c[0][1] : 0.f);
@@ -191,66 +218,54 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
     // weight gradients over the round: dW2t[out][in] = sum_s g2[s][out] h1[s][in]
 #pragma unroll
     for (int kt = 0; kt < kRows / 16; ++kt) {
-      uint32_t b0, b1;
-      b_frag_rows<kMlpH>(S.h1, kt, warp, lane, b0, b1);
+      uint32_t a[4], b[4];
+      b_frag_rows2<kLdH>(S.h1, kt, 2 * warp, lane, b);
 #pragma unroll
       for (int mt = 0; mt < 4; ++mt) {
-        uint32_t a[4];
-        a_frag_t<kMlpH>(S.g2, mt, kt, lane, a);
-        mma_bf16(acc2[mt], a, b0, b1);
+        a_frag_t<kLdH>(S.g2, mt, kt, lane, a);
+        mma_bf16(acc2[mt][0], a, b[0], b[1]);
+        mma_bf16(acc2[mt][1], a, b[2], b[3]);
+        if (mt == warp) mma_bf16(ab2, a, ones, ones);
       }
-      // dW1t[out][in] = sum_s g1[s][out] x[s][in]: warp -> (mt = warp / 2, nt = warp % 2)
-      {
-        uint32_t a[4];
-        a_frag_t<kMlpH>(S.g1, warp >> 1, kt, lane, a);
-        const int nn = 8 * (warp & 1) + g, k0 = 16 * kt + 2 * t;
-        const uint32_t xb0 = pack_bf16(S.x[(size_t)k0 * kMlpIn + nn], S.x[(size_t)(k0 + 1) * kMlpIn + nn]);
-        const uint32_t xb1 = pack_bf16(S.x[(size_t)(k0 + 8) * kMlpIn + nn], S.x[(size_t)(k0 + 9) * kMlpIn + nn]);
-        mma_bf16(acc1, a, xb0, xb1);
-      }
+      // dW1t[out][in] = sum_s g1[s][out] x[s][in]
+      a_frag_t<kLdH>(S.g1, warp, kt, lane, a);
+      b_frag_rows2<kLdX>(S.xb, kt, 0, lane, b);
+      mma_bf16(acc1[0], a, b[0], b[1]);
+      mma_bf16(acc1[1], a, b[2], b[3]);
+      mma_bf16(ab1, a, ones, ones);
       // dW3t[out][hid] = sum_s go[s][out] h2[s][hid]: rows out 0, 1 of the m-tile
-      {
-        uint32_t a[4];
-        a_frag_t<16>(S.go, 0, kt, lane, a);
-        uint32_t hb0, hb1;
-        b_frag_rows<kMlpH>(S.h2, kt, warp, lane, hb0, hb1);
-        mma_bf16(acc3, a, hb0, hb1);
-      }
-    }
-    // bias gradients: column sums
-    if (threadIdx.x < kMlpH) {
-      for (int r = 0; r < kRows; ++r) bacc += __bfloat162float(S.g1[(size_t)r * kMlpH + threadIdx.x]);
-    } else if (threadIdx.x < 2 * kMlpH) {
-      for (int r = 0; r < kRows; ++r) bacc += __bfloat162float(S.g2[(size_t)r * kMlpH + threadIdx.x - kMlpH]);
-    } else if (threadIdx.x < 2 * kMlpH + kMlpOut) {
-      for (int r = 0; r < kRows; ++r) bacc += __bfloat162float(S.go[(size_t)r * 16 + threadIdx.x - 2 * kMlpH]);
+      a_frag_t<kLdX>(S.go, 0, kt, lane, a);
+      b_frag_rows2<kLdH>(S.h2, kt, 2 * warp, lane, b);
+      mma_bf16(acc3[0], a, b[0], b[1]);
+      mma_bf16(acc3[1], a, b[2], b[3]);
+      if (warp == 0) mma_bf16(ab3, a, ones, ones);
     }
   }
   // per-CTA partial gradient
-  float* P = partial + (size_t)blockIdx.x * (kMlpParams + 1);
+  float* P = partial + (size_t)blockIdx.x * kMlpPart;
+  auto put2 = [&](int off, float v0, float v1) {  // the scratch is only known to be 4-byte aligned
+    P[off] = v0;
+    P[off + 1] = v1;
+  };
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt) {
-    const int o = 16 * mt + g, i = 8 * warp + 2 * t;
-    P[kOffW2 + o * kMlpH + i] = acc2[mt][0];
-    P[kOffW2 + o * kMlpH + i + 1] = acc2[mt][1];
-    P[kOffW2 + (o + 8) * kMlpH + i] = acc2[mt][2];
-    P[kOffW2 + (o + 8) * kMlpH + i + 1] = acc2[mt][3];
+  for (int h = 0; h < 2; ++h) {
+    const int i = 8 * (2 * warp + h) + 2 * t;
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+      put2(kOffW2 + (16 * mt + g) * kMlpH + i, acc2[mt][h][0], acc2[mt][h][1]);
+      put2(kOffW2 + (16 * mt + g + 8) * kMlpH + i, acc2[mt][h][2], acc2[mt][h][3]);
+    }
+    put2(kOffW1 + (16 * warp + g) * kMlpIn + 8 * h + 2 * t, acc1[h][0], acc1[h][1]);
+    put2(kOffW1 + (16 * warp + g + 8) * kMlpIn + 8 * h + 2 * t, acc1[h][2], acc1[h][3]);
+    if (g < kMlpOut) put2(kOffW3 + g * kMlpH + i, acc3[h][0], acc3[h][1]);
   }
-  {
-    const int o = 16 * (warp >> 1) + g, i = 8 * (warp & 1) + 2 * t;
-    P[kOffW1 + o * kMlpIn + i] = acc1[0];
-    P[kOffW1 + o * kMlpIn + i + 1] = acc1[1];
-    P[kOffW1 + (o + 8) * kMlpIn + i] = acc1[2];
-    P[kOffW1 + (o + 8) * kMlpIn + i + 1] = acc1[3];
+  if (t == 0) {  // the columns of a product with ones are equal
+    P[kOffB1 + 16 * warp + g] = ab1[0];
+    P[kOffB1 + 16 * warp + g + 8] = ab1[2];
+    P[kOffB2 + 16 * warp + g] = ab2[0];
+    P[kOffB2 + 16 * warp + g + 8] = ab2[2];
+    if (warp == 0 && g < kMlpOut) P[kOffB3 + g] = ab3[0];
   }
-  if (g < kMlpOut) {
-    const int i = 8 * warp + 2 * t;
-    P[kOffW3 + g * kMlpH + i] = acc3[0];
-    P[kOffW3 + g * kMlpH + i + 1] = acc3[1];
-  }
-  if (threadIdx.x < kMlpH) P[kOffB1 + threadIdx.x] = bacc;
-  else if (threadIdx.x < 2 * kMlpH) P[kOffB2 + threadIdx.x - kMlpH] = bacc;
-  else if (threadIdx.x < 2 * kMlpH + kMlpOut) P[kOffB3 + threadIdx.x - 2 * kMlpH] = bacc;
   // loss sum (lanes with t == 0 hold row losses)
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
   if (lane == 0) S.loss[warp] = lsum;
@@ -262,14 +277,30 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
   }
 }
 
-// Sum of the per-CTA partials in CTA order; then either the gradient
-// (grad != nullptr) or one Adam step on prm (m, v moments, step >= 1).
-__global__ void k_mlp_reduce(const float* __restrict__ partial, int nblk, float* grad, float* prm, float* m, float* v,
-                             int step, float lr, float inv_n, float* loss) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > kMlpParams) return;
+// Sum of the per-CTA partials in a fixed order (eight groups of CTAs, then the
+// groups); then either the gradient (grad != nullptr) or one Adam step on prm
+// (m, v moments, step >= 1).  32 parameters per CTA, one group per warp.
+constexpr int kReduceGroups = 8;
+__global__ void __launch_bounds__(32 * kReduceGroups)
+    k_mlp_reduce(const float* __restrict__ partial, int nblk, float* grad, float* prm, float* m, float* v, int step,
+                 float lr, float inv_n, float* loss) {
+  __shared__ float s_sum[kReduceGroups][32];
+  mlp_pdl_trigger();
+  mlp_pdl_wait();
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int b = 0; b < nblk; ++b) s += partial[(size_t)b * (kMlpParams + 1) + i];
+  if (i <= kMlpParams) {
+    const int per = (nblk + kReduceGroups - 1) / kReduceGroups, b0 = grp * per, b1 = min(nblk, b0 + per);
+    const float* p = partial + (size_t)b0 * kMlpPart + i;
+#pragma unroll 8
+    for (int b = b0; b < b1; ++b, p += kMlpPart) s += __ldcg(p);
+  }
+  s_sum[grp][lane] = s;
+  __syncthreads();
+  if (grp != 0 || i > kMlpParams) return;
+  s = 0.f;
+#pragma unroll
+  for (int q = 0; q < kReduceGroups; ++q) s += s_sum[q][lane];
   if (i == kMlpParams) {
     if (loss) *loss = s * inv_n;
     return;
@@ -315,7 +346,25 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_forward(const float* __rest
   }
 }
 
-constexpr int kGradBlocks = 64;
+constexpr int kGradBlocks = 296;  // two CTAs per SM
+
+// Launch that may start while the stream's previous kernel drains (the kernel
+// waits for its results with griddepcontrol.wait).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t lc;
+  memset(&lc, 0, sizeof(lc));
+  lc.gridDim = dim3((unsigned)grid);
+  lc.blockDim = dim3((unsigned)block);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, kernel, args...);
+}
 
 }  // namespace pfb
 
@@ -325,7 +374,7 @@ extern "C" {
 
 int pf_mlp_param_count(void) { return kMlpParams; }
 
-size_t pf_mlp_scratch_bytes(void) { return (size_t)kGradBlocks * (kMlpParams + 1) * sizeof(float); }
+size_t pf_mlp_scratch_bytes(void) { return (size_t)kGradBlocks * kMlpPart * sizeof(float); }
 
 static int grad_launch(const float* d_x, const float* d_y, int n, const float* d_params, float* d_scratch,
                        int* nblk_out, cudaStream_t st) {
@@ -333,8 +382,7 @@ static int grad_launch(const float* d_x, const float* d_y, int n, const float* d
   const size_t smem = sizeof(GradSmem);
   cudaError_t e = cudaFuncSetAttribute((const void*)k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return set_err(PF_ECUDA, "mlp grad attribute: %s", cudaGetErrorString(e));
-  k_mlp_grad<<<nblk, kMlpThreads, smem, st>>>(d_x, d_y, n, d_params, 1.0f / (float)n, d_scratch);
-  e = cudaGetLastError();
+  e = launch_pdl(k_mlp_grad, nblk, kMlpThreads, smem, st, d_x, d_y, n, d_params, 1.0f / (float)n, d_scratch);
   if (e != cudaSuccess) return set_err(PF_ECUDA, "mlp grad launch: %s", cudaGetErrorString(e));
   *nblk_out = nblk;
   return PF_OK;
@@ -349,9 +397,9 @@ int pf_mlp_grad(const float* d_x, const float* d_y, int n, const float* d_params
   cudaStream_t st = (cudaStream_t)stream;
   int nblk = 0, s;
   if ((s = grad_launch(d_x, d_y, n, d_params, (float*)d_scratch, &nblk, st)) != PF_OK) return s;
-  k_mlp_reduce<<<(kMlpParams + 256) / 256, 256, 0, st>>>((const float*)d_scratch, nblk, d_grad, nullptr, nullptr,
-                                                          nullptr, 0, 0.f, 1.0f / (float)n, d_loss);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_pdl(k_mlp_reduce, (kMlpParams + 32) / 32, 32 * kReduceGroups, 0, st, (const float*)d_scratch,
+                             nblk, d_grad, (float*)nullptr, (float*)nullptr, (float*)nullptr, 0, 0.f,
+                             1.0f / (float)n, d_loss);
   return e == cudaSuccess ? PF_OK : set_err(PF_ECUDA, "mlp reduce: %s", cudaGetErrorString(e));
 }
 
@@ -364,9 +412,8 @@ int pf_mlp_adam_step(const float* d_x, const float* d_y, int n, float* d_params,
   cudaStream_t st = (cudaStream_t)stream;
   int nblk = 0, s;
   if ((s = grad_launch(d_x, d_y, n, d_params, (float*)d_scratch, &nblk, st)) != PF_OK) return s;
-  k_mlp_reduce<<<(kMlpParams + 256) / 256, 256, 0, st>>>((const float*)d_scratch, nblk, nullptr, d_params, d_m, d_v,
-                                                          step, lr, 1.0f / (float)n, d_loss);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_pdl(k_mlp_reduce, (kMlpParams + 32) / 32, 32 * kReduceGroups, 0, st, (const float*)d_scratch,
+                             nblk, (float*)nullptr, d_params, d_m, d_v, step, lr, 1.0f / (float)n, d_loss);
   return e == cudaSuccess ? PF_OK : set_err(PF_ECUDA, "mlp adam: %s", cudaGetErrorString(e));
 }
 

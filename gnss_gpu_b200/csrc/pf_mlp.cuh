@@ -12,7 +12,7 @@
 //
 // Why mma.sync and not tcgen05: the network is evaluated per (filter,
 // satellite) -- at most 64 rows per filter and epoch inside the epoch
-// kernel, 128 rows per CTA round in training.  A tcgen05 MMA is 128 rows
+// kernel, 64 rows per CTA round in training.  A tcgen05 MMA is 128 rows
 // wide with its accumulator in TMEM; for these shapes the TMEM allocation,
 // descriptor set-up and round trip would cost more than the math, which is
 // a few hundred register-operand MMAs per CTA.
@@ -53,22 +53,28 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// Row stride of a BF16 matrix of `width` columns in shared memory: 16 bytes
+// more than the row, so that the eight rows a fragment load touches fall into
+// different banks (with rows of exactly 128 bytes every load was an eight-way
+// conflict).
+__host__ __device__ constexpr int mlp_ld(int width) { return width + 8; }
+
 // Weights of one layer as BF16 in shared memory, Wt[out][in] (in
 // contiguous).  The B fragment of k-tile kt, n-tile nt for lane (g, t):
 // b0 = (Wt[n][k], Wt[n][k+1]) with n = 8 nt + g, k = 16 kt + 2t; b1 at k + 8.
 template <int IN>
 __device__ __forceinline__ void b_frag(const __nv_bfloat16* wt, int kt, int nt, int lane, uint32_t& b0, uint32_t& b1) {
   const int g = lane >> 2, t = lane & 3;
-  const __nv_bfloat16* row = wt + (size_t)(8 * nt + g) * IN + 16 * kt + 2 * t;
+  const __nv_bfloat16* row = wt + (8 * nt + g) * mlp_ld(IN) + 16 * kt + 2 * t;
   b0 = *reinterpret_cast<const uint32_t*>(row);
   b1 = *reinterpret_cast<const uint32_t*>(row + 8);
 }
 
 // Network weights staged in shared memory.
 struct MlpSmem {
-  __nv_bfloat16 w1t[kMlpH * kMlpIn];
-  __nv_bfloat16 w2t[kMlpH * kMlpH];
-  __nv_bfloat16 w3t[8 * kMlpH];  // rows 2..7 zero
+  alignas(16) __nv_bfloat16 w1t[kMlpH * mlp_ld(kMlpIn)];
+  alignas(16) __nv_bfloat16 w2t[kMlpH * mlp_ld(kMlpH)];
+  alignas(16) __nv_bfloat16 w3t[8 * mlp_ld(kMlpH)];  // rows 2..7 zero
   float b1[kMlpH];
   float b2[kMlpH];
   float b3[kMlpOut];
@@ -76,10 +82,18 @@ struct MlpSmem {
 
 // All threads of the CTA: FP32 master parameters -> BF16 shared copy.
 __device__ __forceinline__ void mlp_stage(const float* __restrict__ prm, MlpSmem& s, int nthreads) {
-  for (int i = threadIdx.x; i < kMlpH * kMlpIn; i += nthreads) s.w1t[i] = __float2bfloat16_rn(prm[kOffW1 + i]);
-  for (int i = threadIdx.x; i < kMlpH * kMlpH; i += nthreads) s.w2t[i] = __float2bfloat16_rn(prm[kOffW2 + i]);
-  for (int i = threadIdx.x; i < 8 * kMlpH; i += nthreads)
-    s.w3t[i] = __float2bfloat16_rn(i < kMlpOut * kMlpH ? prm[kOffW3 + i] : 0.0f);
+  const uint2 zero = make_uint2(0u, 0u);
+  auto four = [&](int off) {  // the parameter array is only known to be 4-byte aligned
+    return make_uint2(pack_bf16(prm[off], prm[off + 1]), pack_bf16(prm[off + 2], prm[off + 3]));
+  };
+  for (int i = threadIdx.x; i < kMlpH * kMlpIn / 4; i += nthreads)
+    *reinterpret_cast<uint2*>(s.w1t + i / (kMlpIn / 4) * mlp_ld(kMlpIn) + i % (kMlpIn / 4) * 4) = four(kOffW1 + 4 * i);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < kMlpH * kMlpH / 4; i += nthreads)
+    *reinterpret_cast<uint2*>(s.w2t + i / (kMlpH / 4) * mlp_ld(kMlpH) + i % (kMlpH / 4) * 4) = four(kOffW2 + 4 * i);
+  for (int i = threadIdx.x; i < 8 * kMlpH / 4; i += nthreads)
+    *reinterpret_cast<uint2*>(s.w3t + i / (kMlpH / 4) * mlp_ld(kMlpH) + i % (kMlpH / 4) * 4) =
+        i < kMlpOut * kMlpH / 4 ? four(kOffW3 + 4 * i) : zero;
   for (int i = threadIdx.x; i < kMlpH; i += nthreads) {
     s.b1[i] = prm[kOffB1 + i];
     s.b2[i] = prm[kOffB2 + i];
