@@ -42,6 +42,15 @@ __device__ __forceinline__ void write_sat_entry(float2* o, float eE, float eN, f
   o[5] = bc(wq);
 }
 
+// lw -= w rho_k(|r| / sigma) for two particles.
+__device__ __forceinline__ void huber_pair(float2 r, float w, float k, float inv_sigma, float2& lw) {
+  const float z0 = fabsf(r.x) * inv_sigma, z1 = fabsf(r.y) * inv_sigma;
+  const float rho0 = z0 < k ? 0.5f * z0 * z0 : fmaf(k, z0, -0.5f * k * k);
+  const float rho1 = z1 < k ? 0.5f * z1 * z1 : fmaf(k, z1, -0.5f * k * k);
+  lw.x = fmaf(-w, rho0, lw.x);
+  lw.y = fmaf(-w, rho1, lw.y);
+}
+
 // Log-weight update of two particles for one satellite.  With d the
 // particle offset from the anchor, ed = e.d and the receiver clock cb, the
 // range residual to second order in |d|/r0 is
@@ -68,12 +77,7 @@ __device__ __forceinline__ void sat_pair_update(const float2* entry, float2 dx, 
     const float2 rw = __fmul2_rn(r, wq);
     lw = __ffma2_rn(rw, r, lw);
   } else {
-    const float ks = fd->huber_k;
-    const float z0 = fabsf(r.x) * fd->inv_sigma_pr, z1 = fabsf(r.y) * fd->inv_sigma_pr;
-    const float rho0 = z0 < ks ? 0.5f * z0 * z0 : fmaf(ks, z0, -0.5f * ks * ks);
-    const float rho1 = z1 < ks ? 0.5f * z1 * z1 : fmaf(ks, z1, -0.5f * ks * ks);
-    lw.x = fmaf(-wq.x, rho0, lw.x);
-    lw.y = fmaf(-wq.x, rho1, lw.y);
+    huber_pair(r, wq.x, fd->huber_k, fd->inv_sigma_pr, lw);
   }
 }
 

@@ -127,6 +127,58 @@ __device__ __forceinline__ void cta_chunk(int t0, int count, int& b, int& e) {
   chunk_of(t0, count, (int)blockIdx.x, (int)gridDim.x, b, e);
 }
 
+// Phase 1's chunk of this CTA.  With many filters a tile's cost depends on its
+// filter's satellites, so the tiles are cut by cost, not by number: a tile
+// costs kFix + n_sat in units of one satellite, and CTA w takes the tiles whose
+// starts lie in [w, w + 1) / G of the whole cost.  kFix is the rest of a tile
+// (draws, statistics, CDF) over one satellite, fitted to phase 1 of 48 x 100K
+// filters with 8 to 40 satellites (per tile, one clock, us: Gaussian 4.3 + 0.084
+// s, Huber 4.1 + 0.114 s, mixture 4.4 + 0.27 s).  256 filters with 6 to 40
+// satellites: phase 1 ended between 88 and 178 us with equal numbers.
+template <int NCLK, int WMODE>
+__device__ __forceinline__ void weighted_chunk(const EngineDev& e, int t0, int count, const unsigned char* obs0,
+                                               unsigned long long* s_u64, int* s_cut, int& cb, int& ce) {
+  constexpr int kFix = (WMODE == PF_WEIGHT_GAUSSIAN ? 48 : WMODE == PF_WEIGHT_MIXTURE ? 22 : 34) * (NCLK > 1 ? 8 : 5) / 5;
+  const int f0 = __ldg(e.tile_filter + t0), nf = __ldg(e.tile_filter + t0 + count - 1) - f0 + 1;
+  if (nf == 1 || count <= (int)gridDim.x) {  // CTA-uniform
+    cta_chunk(t0, count, cb, ce);
+    return;
+  }
+  const int per = (nf + kThreads - 1) / kThreads, a = min((int)threadIdx.x * per, nf), b = min(a + per, nf);
+  auto tiles_of = [&](int f) {  // of the launch
+    const FilterDesc* fd = e.desc + f;
+    return min(fd->tile_begin + fd->n_tiles, t0 + count) - max(fd->tile_begin, t0);
+  };
+  auto cost_of = [&](int f) {
+    const unsigned epoch = e.ctrl[f].epoch;
+    const pf_filter_epoch_t* fe =
+        reinterpret_cast<const pf_filter_epoch_t*>(obs0 + (size_t)(epoch % (unsigned)e.obs_slots) * e.obs_slot_bytes) + f;
+    return (unsigned long long)(kFix + ((fe->flags & PF_EP_WEIGHT) ? min(max(fe->n_sat, 0), e.max_sats) : 0));
+  };
+  unsigned long long mine = 0, total;
+  for (int k = a; k < b; ++k) mine += cost_of(f0 + k) * (unsigned long long)tiles_of(f0 + k);
+  if (threadIdx.x < 2) s_cut[threadIdx.x] = 0;
+  unsigned long long at = block_excl_scan_u64(mine, s_u64, &total);
+  // tiles that start below each end of the CTA's share
+  const unsigned long long lo = total * blockIdx.x / gridDim.x, hi = total * (blockIdx.x + 1ull) / gridDim.x;
+  int n_lo = 0, n_hi = 0;
+  for (int k = a; k < b; ++k) {
+    const unsigned long long c = cost_of(f0 + k), nt = (unsigned long long)tiles_of(f0 + k);
+    if (lo > at) n_lo += (int)min(nt, (lo - at + c - 1) / c);
+    if (hi > at) n_hi += (int)min(nt, (hi - at + c - 1) / c);
+    at += c * nt;
+  }
+  n_lo = __reduce_add_sync(0xffffffffu, n_lo);
+  n_hi = __reduce_add_sync(0xffffffffu, n_hi);
+  if ((threadIdx.x & 31) == 0) {  // s_cut was cleared before the scan's barriers
+    if (n_lo) atomicAdd(s_cut, n_lo);
+    if (n_hi) atomicAdd(s_cut + 1, n_hi);
+  }
+  __syncthreads();
+  cb = t0 + s_cut[0];
+  ce = t0 + s_cut[1];
+}
+
 // Block-wide sums of two 64-bit values (s_tmp: 2 * kWarps words).
 __device__ __forceinline__ void block_sum2_u64(unsigned long long a, unsigned long long b,
                                                unsigned long long* s_tmp, unsigned long long& ra,
@@ -394,6 +446,7 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
   __shared__ unsigned long long s_u64[2 * kWarps];
   __shared__ double s_wq[kRowBufs][kWarps];  // per-warp sums of the tiled integer CDF
   __shared__ unsigned s_rows[kRowBufs], s_merged[kRowBufs];  // rows written, tiles merged (counts per buffer)
+  __shared__ int s_cut[2];
   __shared__ int s_dec_f, s_dec_rs;  // the filter this CTA owns in phase 2 and its decision
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -404,13 +457,13 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
   unsigned gen = ld_relaxed(bar + 1);
   if (threadIdx.x == 0) s_dec_f = -1;
   if (threadIdx.x < kRowBufs) s_rows[threadIdx.x] = s_merged[threadIdx.x] = 0u;  // ordered by the first table's barriers
-  int cb, ce;
-  cta_chunk(t0, count, cb, ce);
   const unsigned char* const obs0 = in.bytes > 0 ? in.data : e.obs;
   if (in.bytes > 0 && blockIdx.x == gridDim.x - 1)  // slot 0 keeps them for a later step without an upload
     for (int i = threadIdx.x * 8; i < in.bytes; i += kThreads * 8)
       *reinterpret_cast<unsigned long long*>(const_cast<unsigned char*>(e.obs) + i) =
           *reinterpret_cast<const unsigned long long*>(in.data + i);
+  int cb, ce;
+  weighted_chunk<NCLK, WMODE>(e, t0, count, obs0, s_u64, s_cut, cb, ce);
 
   // ---------------------------------------------------------------- phase 1
   int cached = -1;
@@ -555,7 +608,7 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
           nbb[p] = f2(-bb.x, -bb.y);
         }
         if constexpr (WMODE == PF_WEIGHT_GENERIC) {
-          bool gated[4] = {false, false, false, false};
+          float lim[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
           const float gate = e.lk_gate_m;
           if (gate > 0.f) {  // per-particle NLOS gate: drop |r| > gate unless too few satellites remain
             int kept[4] = {0, 0, 0, 0}, used = 0;
@@ -566,13 +619,20 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
             }
             const int need = used < 4 ? used : 4;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) gated[k] = kept[k] >= need;
+            for (int k = 0; k < 4; ++k) lim[k] = kept[k] >= need ? gate : INFINITY;
           }
+          auto all_clocks = [&](auto type) {
 #pragma unroll
-          for (int c = 0; c < NCLK; ++c) {
-            const float2 ncb[2] = {f2(-x[3 + c][0], -x[3 + c][1]), f2(-x[3 + c][2], -x[3 + c][3])};
-            generic_pairs(s_sat, s_grp[c], s_grp[c + 1], dx, dy, dz, nbb, ncb, lwp, gated, gate);
-          }
+            for (int c = 0; c < NCLK; ++c) {
+              const float2 ncb[2] = {f2(-x[3 + c][0], -x[3 + c][1]), f2(-x[3 + c][2], -x[3 + c][3])};
+              generic_pairs<decltype(type)::value>(s_sat, s_grp[c], s_grp[c + 1], dx, dy, dz, nbb, ncb, lwp, lim,
+                                                   e.lk_huber_k, fd->inv_sigma_pr, -0.5f * (e.lk_nu + 1.f));
+            }
+          };
+          if (e.lk_type == PF_LIK_STUDENT_T) all_clocks(LikType<PF_LIK_STUDENT_T>());
+          else if (e.lk_type == PF_LIK_HUBER) all_clocks(LikType<PF_LIK_HUBER>());
+          else if (e.lk_type == PF_LIK_GMM) all_clocks(LikType<PF_LIK_GMM>());
+          else all_clocks(LikType<PF_LIK_GAUSSIAN>());
         }
 #pragma unroll
         for (int c = 0; c < NCLK && WMODE != PF_WEIGHT_GENERIC; ++c) {
@@ -700,6 +760,7 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
     // the snapshot phase 1 left (the owner advances the epoch meanwhile).
     int cf = -1;
     bool crs = false;
+    cta_chunk(t0, count, cb, ce);  // here every tile costs the same
     for (int t = cb; t < ce; ++t) {
       const int f = __ldg(e.tile_filter + t);
       const FilterDesc* fd = e.desc + f;

@@ -14,9 +14,11 @@
 // The residual r is the epoch kernel's second-order form (sat_pair_update).
 // Satellite table entries use the mixture layout (kMixStride float2):
 //   eE eN | eU g/2 | y w | c0 c1 | c2 c3 | mu mode
-// mode 0 GMM (c0 = log w_los - log sigma, c1 = -w/(2 sigma^2), c2, c3 the
-// NLOS pair), 1 Huber (c0 = k, c1 = 1/sigma), 2 unused, 3 Student's t
-// (c0 = -(nu+1)/2, c1 = w/(nu sigma^2)), 4 Gaussian (c1 = -w/(2 sigma^2)).
+// GMM: c0 = log w_los - log sigma, c1 = -w / (2 sigma^2), c2, c3 the NLOS pair, -mu
+// in the place of mu; Huber: none; Student's t: c1 = w / (nu
+// sigma^2); Gaussian: c1 = -w / (2 sigma^2).  One likelihood holds for every
+// satellite, and one of weight <= 0 gets constants that add nothing, so the loops
+// are free of branches.
 #pragma once
 #include "pf_learned.cuh"
 
@@ -25,33 +27,29 @@ namespace pfb {
 // Table entry of one satellite for the generic likelihood.
 __device__ __forceinline__ void write_generic_entry(float2* o, const EngineDev& e, float sigma, float eE, float eN,
                                                     float eU, float g, float y, float w) {
+  const bool used = w > 0.f;
   o[0] = bc(eE); o[1] = bc(eN); o[2] = bc(eU); o[3] = bc(0.5f * g);
-  o[4] = bc(y); o[5] = bc(w);
-  float mode = 4.f, c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f, mu = 0.f;
+  o[4] = bc(y); o[5] = bc(used ? w : 0.f);
+  float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f, mu = 0.f;
   const float s2 = sigma * sigma;
-  if (!(w > 0.f)) {
-    mode = 2.f;
-  } else if (e.lk_type == PF_LIK_STUDENT_T) {
-    mode = 3.f;
-    c0 = -0.5f * (e.lk_nu + 1.f);
-    c1 = w / (e.lk_nu * s2);
-  } else if (e.lk_type == PF_LIK_HUBER) {
-    mode = 1.f;
-    c0 = e.lk_huber_k;
-    c1 = 1.f / sigma;
-  } else if (e.lk_type == PF_LIK_GMM) {
-    mode = 0.f;
+  if (e.lk_type == PF_LIK_GMM) {
     const float sn = e.lk_sigma_nlos;
-    c0 = logf(e.lk_w_los) - logf(sigma);
-    c1 = -0.5f * w / s2;
-    c2 = logf(1.f - e.lk_w_los) - logf(sn);
-    c3 = -0.5f * w / (sn * sn);
-    mu = e.lk_mu_nlos;
-  } else {
+    c2 = -INFINITY;  // unused: log(e^0 + 0)
+    if (used) {
+      c0 = logf(e.lk_w_los) - logf(sigma);
+      c1 = -0.5f * w / s2;
+      c2 = logf(1.f - e.lk_w_los) - logf(sn);
+      c3 = -0.5f * w / (sn * sn);
+      mu = e.lk_mu_nlos;
+    }
+  } else if (!used) {
+  } else if (e.lk_type == PF_LIK_STUDENT_T) {
+    c1 = w / (e.lk_nu * s2);
+  } else if (e.lk_type == PF_LIK_GAUSSIAN) {
     c1 = -0.5f * w / s2;
   }
   o[6] = bc(c0); o[7] = bc(c1); o[8] = bc(c2); o[9] = bc(c3);
-  o[10] = bc(mu); o[11] = bc(mode);
+  o[10] = bc(-mu); o[11] = bc(0.f);
 }
 
 // Residual of two particles for one table entry (as sat_pair_update).
@@ -69,38 +67,47 @@ __device__ __forceinline__ float2 entry_residual(const float2* entry, float2 dx,
   return __ffma2_rn(sq, g2, ye);
 }
 
-// Log-likelihood term of one satellite for one particle.
-__device__ __forceinline__ float generic_term(const float4 q3, const float4 q4, const float4 q5, float w, float r) {
-  const float mode = q5.z;
-  if (mode > 3.5f) return q3.z * r * r;                              // Gaussian
-  if (mode > 2.5f) return q3.x * __logf(fmaf(q3.z * r, r, 1.f));     // Student's t
-  if (mode > 0.5f) {                                                  // Huber
-    const float z = fabsf(r) * q3.z, k = q3.x;
-    return -w * (z < k ? 0.5f * z * z : fmaf(k, z, -0.5f * k * k));
-  }
-  const float a = fmaf(q3.z * r, r, q3.x);                            // GMM
-  const float dm = r - q5.x;
-  const float b = fmaf(q4.z * dm, dm, q4.x);
-  const float hi = fmaxf(a, b), lo = fminf(a, b);
-  return hi + __logf(1.f + __expf(lo - hi));
-}
+template <int T>
+struct LikType {
+  static constexpr int value = T;
+};
 
-// Adds the satellites [s0, s1) of the table to the log-weights of two
-// particle pairs (with the per-particle gate when gate > 0).
+// Adds the satellites [s0, s1) of the table to two particle pairs; a residual
+// beyond lim[k] (infinite without the gate) is dropped.
+template <int TYPE>
 __device__ __forceinline__ void generic_pairs(const float2* s_sat, int s0, int s1, const float2 (&dx)[2],
                                               const float2 (&dy)[2], const float2 (&dz)[2], const float2 (&nbb)[2],
-                                              const float2 (&ncb)[2], float2 (&lwp)[2], bool (&gated)[4],
-                                              float gate) {
+                                              const float2 (&ncb)[2], float2 (&lwp)[2], const float (&lim)[4],
+                                              float huber_k, float inv_sigma, float t_scale) {
+#pragma unroll 2
   for (int s = s0; s < s1; ++s) {
     const float2* entry = s_sat + kMixStride * s;
     const float4* sv = reinterpret_cast<const float4*>(entry);
-    const float4 q2 = sv[2], q3 = sv[3], q4 = sv[4], q5 = sv[5];
-    if (q5.z > 1.5f && q5.z < 2.5f) continue;  // weight 0
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       const float2 r = entry_residual(entry, dx[p], dy[p], dz[p], nbb[p], ncb[p]);
-      if (!(gated[2 * p] && fabsf(r.x) > gate)) lwp[p].x += generic_term(q3, q4, q5, q2.z, r.x);
-      if (!(gated[2 * p + 1] && fabsf(r.y) > gate)) lwp[p].y += generic_term(q3, q4, q5, q2.z, r.y);
+      const bool o0 = fabsf(r.x) > lim[2 * p], o1 = fabsf(r.y) > lim[2 * p + 1];
+      if constexpr (TYPE == PF_LIK_GAUSSIAN) {
+        const float4 q3 = sv[3];
+        const float2 rk = f2(o0 ? 0.f : r.x, o1 ? 0.f : r.y);
+        lwp[p] = __ffma2_rn(__fmul2_rn(f2(q3.z, q3.w), rk), rk, lwp[p]);
+      } else if constexpr (TYPE == PF_LIK_HUBER) {
+        const float4 q2 = sv[2];
+        huber_pair(f2(o0 ? 0.f : r.x, o1 ? 0.f : r.y), q2.z, huber_k, inv_sigma, lwp[p]);
+      } else if constexpr (TYPE == PF_LIK_STUDENT_T) {
+        const float4 q3 = sv[3];
+        const float2 rk = f2(o0 ? 0.f : r.x, o1 ? 0.f : r.y);
+        const float2 q = __ffma2_rn(__fmul2_rn(f2(q3.z, q3.w), rk), rk, bc(1.f));  // >= 1
+        lwp[p] = __ffma2_rn(bc(t_scale), __fmul2_rn(f2(lg2_normal(q.x), lg2_normal(q.y)), bc(0.693147180559945309f)),
+                            lwp[p]);
+      } else {
+        const float4 q3 = sv[3], q4 = sv[4], q5 = sv[5];
+        const float2 a = __ffma2_rn(__fmul2_rn(f2(q3.z, q3.w), r), r, f2(q3.x, q3.y));
+        const float2 dm = __fadd2_rn(r, f2(q5.x, q5.y));
+        const float2 b = __ffma2_rn(__fmul2_rn(f2(q4.z, q4.w), dm), dm, f2(q4.x, q4.y));
+        const float2 l = log_add_pair(a, b);
+        lwp[p] = __fadd2_rn(lwp[p], f2(o0 ? 0.f : l.x, o1 ? 0.f : l.y));
+      }
     }
   }
 }

@@ -182,7 +182,7 @@ __device__ __forceinline__ void build_mixture_table(const EngineDev& e, const Fi
     o[0] = bc(eE); o[1] = bc(eN); o[2] = bc(eU); o[3] = bc(0.5f * g);
     o[4] = bc(y); o[5] = bc((float)w);
     o[6] = bc(ca); o[7] = bc(ia); o[8] = bc(cb); o[9] = bc(ib);
-    o[10] = bc(mu); o[11] = bc(mode);
+    o[10] = bc(-mu); o[11] = bc(mode);
     if (export_dbg) {
       float* d = e.sat_dbg + ((size_t)f * e.max_sats + s) * kSatDbg;
 #pragma unroll
@@ -200,6 +200,22 @@ __device__ __forceinline__ void build_mixture_table(const EngineDev& e, const Fi
     s_grp[threadIdx.x] = cnt;
   }
   __syncthreads();
+}
+
+// log(e^a + e^b) of two particles: max + log(1 + e^-|a - b|), packed but for
+// the maximum and the MUFU operations, and these without subnormal handling
+// (e^-|a - b| below 2^-126 adds nothing to 1, 1 + e^-|a - b| is in [1, 2]).
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 log_add_pair(float2 a, float2 b) {
+  const float2 d = __ffma2_rn(b, bc(-1.0f), a);
+  const float2 t = __fadd2_rn(f2(ex2_ftz(-1.4426950408889634f * fabsf(d.x)), ex2_ftz(-1.4426950408889634f * fabsf(d.y))),
+                              bc(1.0f));
+  return __ffma2_rn(f2(lg2_normal(t.x), lg2_normal(t.y)), bc(0.693147180559945309f),
+                    f2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)));
 }
 
 // Log-likelihood update of two particles for one satellite in mixture mode
@@ -220,25 +236,15 @@ __device__ __forceinline__ void sat_pair_mixture(const float2* entry, float2 dx,
   const float2 sq = __ffma2_rn(ed, ed, nbb);
   const float2 r = __ffma2_rn(sq, g2, ye);
   if (mode > 0.5f) {  // Huber fallback (uniform over the warp: one satellite at a time)
-    const float wq = q2.z;
-    const float ks = fd->huber_k;
-    const float z0 = fabsf(r.x) * fd->inv_sigma_pr, z1 = fabsf(r.y) * fd->inv_sigma_pr;
-    const float rho0 = z0 < ks ? 0.5f * z0 * z0 : fmaf(ks, z0, -0.5f * ks * ks);
-    const float rho1 = z1 < ks ? 0.5f * z1 * z1 : fmaf(ks, z1, -0.5f * ks * ks);
-    lw.x = fmaf(-wq, rho0, lw.x);
-    lw.y = fmaf(-wq, rho1, lw.y);
+    huber_pair(r, q2.z, fd->huber_k, fd->inv_sigma_pr, lw);
     return;
   }
   const float4 q3 = sv[3], q4 = sv[4];
   const float2 ca = f2(q3.x, q3.y), ia = f2(q3.z, q3.w), cb = f2(q4.x, q4.y), ib = f2(q4.z, q4.w);
-  const float2 mu = f2(q5.x, q5.y);
   const float2 a = __ffma2_rn(__fmul2_rn(r, r), ia, ca);
-  const float2 dm = __ffma2_rn(mu, bc(-1.0f), r);
+  const float2 dm = __fadd2_rn(r, f2(q5.x, q5.y));
   const float2 b = __ffma2_rn(__fmul2_rn(dm, dm), ib, cb);
-  const float hi0 = fmaxf(a.x, b.x), lo0 = fminf(a.x, b.x);
-  const float hi1 = fmaxf(a.y, b.y), lo1 = fminf(a.y, b.y);
-  lw.x += hi0 + __logf(1.0f + __expf(lo0 - hi0));
-  lw.y += hi1 + __logf(1.0f + __expf(lo1 - hi1));
+  lw = __fadd2_rn(lw, log_add_pair(a, b));
 }
 
 }  // namespace pfb
