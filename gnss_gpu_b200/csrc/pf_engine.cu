@@ -1576,13 +1576,11 @@ int pfe_add_obs_term(pf_engine_t* eng, int filter, int kind, const pf_obs_row_t*
   b.huber_k = huber_k;
   if (n_rows > 0)
     CK(cudaMemcpyAsync(eng->obs_rows, host.data(), sizeof(ObsRow) * n_rows, cudaMemcpyHostToDevice, eng->stream));
-  const int g = std::max(1, std::min(eng->sm_count * 4, (d.n + kTile - 1) / kTile));
-  switch (eng->D) {
-    case 4: k_obs_term<4><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, b, eng->obs_rows); break;
-    case 5: k_obs_term<5><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, b, eng->obs_rows); break;
-    case 6: k_obs_term<6><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, b, eng->obs_rows); break;
-    default: k_obs_term<7><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, b, eng->obs_rows); break;
-  }
+  const int g = std::max(1, std::min(eng->sm_count * 16, (d.n + kThreads - 1) / kThreads));
+  const auto term = kind == PF_OBS_DD_PSEUDORANGE ? k_obs_term<PF_OBS_DD_PSEUDORANGE>
+                    : kind == PF_OBS_CARRIER_AFV  ? k_obs_term<PF_OBS_CARRIER_AFV>
+                                                  : k_obs_term<PF_OBS_DD_CARRIER_AFV>;
+  term<<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, b, eng->obs_rows);
   CK(cudaGetLastError());
   const int zero = 0;
   CK(cudaMemcpyAsync(reinterpret_cast<char*>(eng->ctrl_dev + filter) + offsetof(FilterCtrl, lw_zero), &zero,
