@@ -1118,14 +1118,21 @@ static int run_estimate(pf_engine_t* eng, int filter) {
   if (!eng->initialized[filter]) return set_err(PF_ENOTINIT, "filter %d not initialized", filter);
   const FilterDesc& d = eng->hdesc[filter];
   const int g = grid_for(eng, Q_EST, d.n_tiles);
+  EngineDev dev = eng->dev;
+  dev.err_map = eng->err_host;
+  *eng->err_host = 0u;
+  FilterCtrl* out = eng->ctrl_host + filter;
   switch (eng->D) {
-    case 4: k_estimate<4><<<g, kThreads, 0, eng->stream>>>(eng->dev, d.tile_begin, d.n_tiles); break;
-    case 5: k_estimate<5><<<g, kThreads, 0, eng->stream>>>(eng->dev, d.tile_begin, d.n_tiles); break;
-    case 6: k_estimate<6><<<g, kThreads, 0, eng->stream>>>(eng->dev, d.tile_begin, d.n_tiles); break;
-    default: k_estimate<7><<<g, kThreads, 0, eng->stream>>>(eng->dev, d.tile_begin, d.n_tiles); break;
+    case 4: k_estimate<4><<<g, kThreads, 0, eng->stream>>>(dev, d.tile_begin, d.n_tiles, out); break;
+    case 5: k_estimate<5><<<g, kThreads, 0, eng->stream>>>(dev, d.tile_begin, d.n_tiles, out); break;
+    case 6: k_estimate<6><<<g, kThreads, 0, eng->stream>>>(dev, d.tile_begin, d.n_tiles, out); break;
+    default: k_estimate<7><<<g, kThreads, 0, eng->stream>>>(dev, d.tile_begin, d.n_tiles, out); break;
   }
   CK(cudaGetLastError());
-  return read_ctrl(eng);
+  CK(cudaStreamSynchronize(eng->stream));
+  if (*(volatile unsigned*)eng->err_host)
+    CK(cudaMemcpy(eng->err_host, eng->dev.err, sizeof(unsigned), cudaMemcpyDeviceToHost));
+  return err_status(*eng->err_host);
 }
 
 int pfe_estimate(pf_engine_t* eng, int filter, double* out) {

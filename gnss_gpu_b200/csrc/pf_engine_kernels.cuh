@@ -1404,9 +1404,11 @@ __global__ void __launch_bounds__(kThreads) k_init(EngineDev e, int t0, int coun
 // log-weights (zeros after a resample) -- the reference's pf_estimate
 // semantics (weight.cu:163-220,301-321) -- plus the ESS of those weights
 // (pf_device.cu:924) and the weighted second moments of the local position
-// offsets (for the position spread, pf_device.cu:1025).
+// offsets (for the position spread, pf_device.cu:1025).  The results also go
+// straight into `out`, the host's pinned mirror of the control block, with the
+// anchor: the caller waits for the kernel alone, not for a copy after it.
 template <int D>
-__global__ void __launch_bounds__(kThreads) k_estimate(EngineDev e, int t0, int count) {
+__global__ void __launch_bounds__(kThreads) k_estimate(EngineDev e, int t0, int count, FilterCtrl* out) {
   __shared__ float s_red[kThreads / 32][kPartStride];
   __shared__ float s_maxtmp[kThreads / 32];
   __shared__ double s_dred[(kThreads / 32) * 16];
@@ -1459,14 +1461,22 @@ __global__ void __launch_bounds__(kThreads) k_estimate(EngineDev e, int t0, int 
         const double W = ms.w;
         double est[3];
         local_to_ecef(fd->rot, fc->anchor, ms.sx[0] / W, ms.sx[1] / W, ms.sx[2] / W, est);
-        fc->api_est[0] = est[0];
-        fc->api_est[1] = est[1];
-        fc->api_est[2] = est[2];
+        FilterCtrl* dst[2] = {fc, out};
 #pragma unroll
-        for (int c = 0; c < D - 3; ++c) fc->api_est[3 + c] = fc->clk_anchor[c] + ms.sx[3 + c] / W;
-        fc->api_est[7] = (ms.w2 > 0.0) ? W * W / ms.w2 : 0.0;
+        for (int w = 0; w < 2; ++w) {
+          FilterCtrl* o = dst[w];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) fc->api_m2[i] = ms.sxx[i] / W;
+          for (int i = 0; i < 3; ++i) o->api_est[i] = est[i];
+#pragma unroll
+          for (int c = 0; c < D - 3; ++c) o->api_est[3 + c] = fc->clk_anchor[c] + ms.sx[3 + c] / W;
+          o->api_est[7] = (ms.w2 > 0.0) ? W * W / ms.w2 : 0.0;
+#pragma unroll
+          for (int i = 0; i < 6; ++i) o->api_m2[i] = ms.sxx[i] / W;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) out->anchor[i] = fc->anchor[i];
+        const unsigned err = *(volatile unsigned*)e.err;
+        if (err) *(volatile unsigned*)e.err_map = err;
         fc->est_ticket = 0u;
         __threadfence();
       }
