@@ -1646,10 +1646,23 @@ int pfe_vel_follow(pf_engine_t* eng, int filter, pf_vel_state_t* vs) {
   return sync_and_check(eng);
 }
 
+}  // extern "C"
+
+namespace {
+template <int D>
+void launch_vel_predict(pf_engine* eng, int filter, const double* vin, double* vout, const VelPredict& vp) {
+  const int g = std::max(1, std::min(eng->sm_count * 16, (eng->hdesc[filter].n + kThreads - 1) / kThreads));
+  if (vp.kf) k_vel_predict<D, true><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vin, vout, vp);
+  else k_vel_predict<D, false><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vin, vout, vp);
+}
+}  // namespace
+
+extern "C" {
+
 int pfe_vel_predict(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const double guide_ecef[3], double dt,
                     double sigma_pos, double sigma_vel, double alpha, int kf, double q, unsigned step) {
   clear_err();
-  int s = pfe_vel_follow(eng, filter, vs);
+  int s = vel_check(eng, filter, vs);
   if (s != PF_OK) return s;
   if (!guide_ecef) return set_err(PF_EINVAL, "null guide velocity");
   for (int i = 0; i < 3; ++i)
@@ -1657,7 +1670,8 @@ int pfe_vel_predict(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const doub
   if (!isfinite(dt) || !isfinite(sigma_pos) || !isfinite(sigma_vel) || !isfinite(alpha) || !isfinite(q) ||
       sigma_pos < 0.0 || sigma_vel < 0.0)
     return set_err(PF_EINVAL, "predict parameters must be finite, sigmas >= 0");
-  FilterCtrl c = eng->ctrl_host[filter];  // read by the follow above
+  if ((s = read_ctrl(eng)) != PF_OK) return s;
+  FilterCtrl& c = eng->ctrl_host[filter];
   const FilterDesc& d = eng->hdesc[filter];
   VelPredict vp;
   memset(&vp, 0, sizeof(vp));
@@ -1670,21 +1684,23 @@ int pfe_vel_predict(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const doub
   vp.q = q;
   vp.kf = kf ? 1 : 0;
   vp.step = step;
-  double* vb = vs->buf + (size_t)vs->sel * kVelComp * d.n;
-  const int g = vel_grid(eng, d.n, 4);
-  switch (eng->D) {
-    case 4: k_vel_predict<4><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vb, vp); break;
-    case 5: k_vel_predict<5><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vb, vp); break;
-    case 6: k_vel_predict<6><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vb, vp); break;
-    default: k_vel_predict<7><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, vb, vp); break;
+  // a resample the velocity states have not followed yet is applied on the way
+  const double* vin = vs->buf + (size_t)vs->sel * kVelComp * d.n;
+  if (c.resample_flag && c.rs_seq != vs->seq) {
+    vs->sel ^= 1;
+    vs->seq = c.rs_seq;
   }
+  double* vout = vs->buf + (size_t)vs->sel * kVelComp * d.n;
+  switch (eng->D) {
+    case 4: launch_vel_predict<4>(eng, filter, vin, vout, vp); break;
+    case 5: launch_vel_predict<5>(eng, filter, vin, vout, vp); break;
+    case 6: launch_vel_predict<6>(eng, filter, vin, vout, vp); break;
+    default: launch_vel_predict<7>(eng, filter, vin, vout, vp); break;
+  }
+  k_flip_state<<<1, 1, 0, eng->stream>>>(eng->ctrl_dev + filter);
   CK(cudaGetLastError());
-  // the particles now sit, gathered, in the other buffer
   c.parity ^= 1;
   c.resample_flag = 0;
-  CK(cudaMemcpyAsync(eng->ctrl_dev + filter, &c, sizeof(c), cudaMemcpyHostToDevice, eng->stream));
-  CK(cudaStreamSynchronize(eng->stream));
-  eng->ctrl_host[filter] = c;
   return sync_and_check(eng);
 }
 

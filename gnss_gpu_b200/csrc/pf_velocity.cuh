@@ -94,67 +94,98 @@ struct VelPredict {
 // sigma_pos^2 I + dt^2 P_v) (Cholesky) in KF mode, else N(0, sigma_pos^2 I);
 // KF mode adds q * dt to the velocity variances.  The positions are read
 // through the pending resample gather and written to the other state
-// buffer (the caller flips the parity); clocks are copied.
-template <int D>
-__global__ void __launch_bounds__(kThreads) k_vel_predict(EngineDev e, int f, double* vb, VelPredict vp) {
+// buffer (k_flip_state follows); clocks are copied.
+//
+// The velocity states follow a pending resample in the same pass (vin != vout:
+// read at the ancestor, written in place), so they cross HBM once instead of
+// twice, and only the normals in use are drawn.  One particle per thread.  1M
+// particles with sampled velocities, gather and predict: 66 -> 43 us; 300K with
+// the Kalman covariance 28 -> 14 us.
+template <int D, bool KF>
+__global__ void __launch_bounds__(kThreads) k_vel_predict(EngineDev e, int f, const double* vin, double* vout,
+                                                         VelPredict vp) {
   const FilterDesc* fd = e.desc + f;
   const FilterCtrl* fc = e.ctrl + f;
-  const int n = fd->n;
-  const long long base = fd->p_off;
-  const float* src = fc->parity ? e.state1 : e.state0;
-  float* dst = fc->parity ? e.state0 : e.state1;
+  const ParticleSrc ps = particle_src(e, fd, fc);
+  const int n = ps.n;
+  float* dst = (fc->parity ? e.state0 : e.state1) + ps.base;
   const double alpha = fmin(1.0, fmax(0.0, vp.alpha));
-  for (int p0 = (blockIdx.x * kThreads + threadIdx.x) * 4; p0 < n; p0 += gridDim.x * kThreads * 4) {
-    float x[D][4];
-    load_particles<D>(e, fd, src, base, p0, n, fc->resample_flag != 0, x);
-#pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-      const int j = p0 + k;
-      if (j >= n) break;
-      double z[8];
-      vel_normals((uint32_t)j, vp.step, TAG_VEL_PREDICT, fd, z);
-      double v[3];
-      for (int i = 0; i < 3; ++i) v[i] = (1.0 - alpha) * vb[(size_t)i * n + j] + alpha * vp.guide[i];
-      int zi = 0;
-      if (!vp.kf && vp.sigma_vel > 0.0)
-        for (int i = 0; i < 3; ++i) v[i] += z[zi++] * vp.sigma_vel;
-      for (int i = 0; i < 3; ++i) vb[(size_t)i * n + j] = v[i];
-      double nz[3];
-      if (vp.kf) {
-        double P[9];
-        for (int c = 0; c < 9; ++c) P[c] = vb[(size_t)(3 + c) * n + j];
-        const double dt2 = vp.dt * vp.dt, s2 = vp.sigma_pos * vp.sigma_pos;
-        const double a00 = s2 + dt2 * P[0], a01 = dt2 * P[1], a02 = dt2 * P[2];
-        const double a11 = s2 + dt2 * P[4], a12 = dt2 * P[5], a22 = s2 + dt2 * P[8];
-        const double l00 = sqrt(fmax(a00, 0.0));
-        double l10 = 0.0, l20 = 0.0;
-        if (l00 > 1e-12) {
-          l10 = a01 / l00;
-          l20 = a02 / l00;
-        }
-        const double l11 = sqrt(fmax(a11 - l10 * l10, 0.0));
-        double l21 = 0.0;
-        if (l11 > 1e-12) l21 = (a12 - l20 * l10) / l11;
-        const double l22 = sqrt(fmax(a22 - l20 * l20 - l21 * l21, 0.0));
-        nz[0] = l00 * z[0];
-        nz[1] = l10 * z[0] + l11 * z[1];
-        nz[2] = l20 * z[0] + l21 * z[1] + l22 * z[2];
-        const double qdt = fmax(vp.q, 0.0) * fmax(vp.dt, 0.0);
-        vb[(size_t)3 * n + j] = P[0] + qdt;
-        vb[(size_t)7 * n + j] = P[4] + qdt;
-        vb[(size_t)11 * n + j] = P[8] + qdt;
-      } else {
-        for (int i = 0; i < 3; ++i) nz[i] = z[zi++] * vp.sigma_pos;
-      }
-      double d[3];
-      for (int i = 0; i < 3; ++i) d[i] = v[i] * vp.dt + nz[i];
-      for (int r = 0; r < 3; ++r)
-        x[r][k] = (float)((double)x[r][k] + vp.rot[3 * r] * d[0] + vp.rot[3 * r + 1] * d[1] + vp.rot[3 * r + 2] * d[2]);
+  const bool noisy = !KF && vp.sigma_vel > 0.0, moved = vin != vout;
+  for (int j = blockIdx.x * kThreads + threadIdx.x; j < n; j += gridDim.x * kThreads) {
+    const float* sp = particle_at(e, ps, j);
+    const int a = moved ? (int)(sp - (ps.src + ps.base)) : j;
+    float x[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) x[d] = __ldcg(sp + (size_t)d * e.p_total);
+    double v[3], P[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v[i] = vin[(size_t)i * n + a];
+    if (KF || moved)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) P[c] = vin[(size_t)(3 + c) * n + a];
+    double z[6];
+    const U4 r0 = philox10(U4{(uint32_t)j, vp.step, TAG_VEL_PREDICT, (uint32_t)fd->filter_id}, fd->key0, fd->key1);
+    normals2_f64(r0.x, r0.y, z[0], z[1]);
+    normals2_f64(r0.z, r0.w, z[2], z[3]);
+    if (noisy) {
+      const U4 r1 = philox10(U4{(uint32_t)j, vp.step, TAG_VEL_PREDICT | 1u, (uint32_t)fd->filter_id}, fd->key0, fd->key1);
+      normals2_f64(r1.x, r1.y, z[4], z[5]);
     }
 #pragma unroll
-    for (int d = 0; d < D; ++d)
-      *reinterpret_cast<float4*>(dst + (size_t)d * e.p_total + base + p0) = make_float4(x[d][0], x[d][1], x[d][2], x[d][3]);
+    for (int i = 0; i < 3; ++i) {
+      v[i] = (1.0 - alpha) * v[i] + alpha * vp.guide[i];
+      if (noisy) v[i] += z[i] * vp.sigma_vel;
+      vout[(size_t)i * n + j] = v[i];
+    }
+    double nz[3];
+    if constexpr (KF) {
+      const double dt2 = vp.dt * vp.dt, s2 = vp.sigma_pos * vp.sigma_pos;
+      const double a00 = s2 + dt2 * P[0], a01 = dt2 * P[1], a02 = dt2 * P[2];
+      const double a11 = s2 + dt2 * P[4], a12 = dt2 * P[5], a22 = s2 + dt2 * P[8];
+      const double l00 = sqrt(fmax(a00, 0.0));
+      double l10 = 0.0, l20 = 0.0;
+      if (l00 > 1e-12) {
+        l10 = a01 / l00;
+        l20 = a02 / l00;
+      }
+      const double l11 = sqrt(fmax(a11 - l10 * l10, 0.0));
+      double l21 = 0.0;
+      if (l11 > 1e-12) l21 = (a12 - l20 * l10) / l11;
+      const double l22 = sqrt(fmax(a22 - l20 * l20 - l21 * l21, 0.0));
+      nz[0] = l00 * z[0];
+      nz[1] = l10 * z[0] + l11 * z[1];
+      nz[2] = l20 * z[0] + l21 * z[1] + l22 * z[2];
+      const double qdt = fmax(vp.q, 0.0) * fmax(vp.dt, 0.0);
+      P[0] += qdt;
+      P[4] += qdt;
+      P[8] += qdt;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) nz[i] = (noisy ? z[3 + i] : z[i]) * vp.sigma_pos;
+    }
+    if (moved) {
+#pragma unroll
+      for (int c = 0; c < 9; ++c) vout[(size_t)(3 + c) * n + j] = P[c];
+    } else if constexpr (KF) {
+      vout[(size_t)3 * n + j] = P[0];
+      vout[(size_t)7 * n + j] = P[4];
+      vout[(size_t)11 * n + j] = P[8];
+    }
+    double d[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) d[i] = v[i] * vp.dt + nz[i];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+      x[r] = (float)((double)x[r] + vp.rot[3 * r] * d[0] + vp.rot[3 * r + 1] * d[1] + vp.rot[3 * r + 2] * d[2]);
+#pragma unroll
+    for (int d2 = 0; d2 < D; ++d2) dst[(size_t)d2 * e.p_total + j] = x[d2];
   }
+}
+
+// The particles now sit, gathered, in the other state buffer.
+__global__ void k_flip_state(FilterCtrl* fc) {
+  fc->parity ^= 1;
+  fc->resample_flag = 0;
 }
 
 // ECEF position of local offsets (x, y, z) about the filter's anchor.
