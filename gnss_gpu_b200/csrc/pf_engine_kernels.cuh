@@ -1533,6 +1533,18 @@ __global__ void __launch_bounds__(kThreads) k_position_term(EngineDev e, int f, 
   }
 }
 
+// The end of a call that wrote log-weights: they are explicit now, and the error
+// word goes to its pinned mirror.
+__global__ void k_term_done(FilterCtrl* fc, const unsigned* err, unsigned* err_map) {
+  fc->lw_zero = 0;
+  *err_map = *err;
+}
+
+// Control blocks and error word to their pinned mirror (words of 4 bytes).
+__global__ void __launch_bounds__(kThreads) k_mirror(const unsigned* src, unsigned* dst, int words) {
+  for (int i = threadIdx.x; i < words; i += kThreads) dst[i] = src[i];
+}
+
 // -------------------------------------------------------------------------
 // k_export: current particles as FP64 ECEF rows [n][D] (x, y, z, clocks),
 // the reference's pf_get_particles layout (weight.cu:331-340).

@@ -10,9 +10,9 @@
 // rows with |r| > gate are dropped unless fewer than min(n, 3) would remain.
 //
 // Carrier terms resolve centimetres out of 2e7 m ranges, so this kernel
-// works in FP64 (the FP32 offsets are exact in FP64; satellites are given
-// in the filter's local frame about its anchor, computed on the host in
-// FP64).  Each row's constant part is folded on the host:
+// works in FP64 (the FP32 offsets are exact in FP64).  The rows arrive as a
+// kernel parameter in ECEF; every CTA takes them to the filter's local frame
+// about its anchor and folds each row's constant part:
 //   DD pseudorange    c = dd + b_k - b_ref,               r = c - (r_k - r_ref)
 //   carrier           c = cp - clk_anchor / lambda,       a = afv(c - (r + x_clk) / lambda)
 //   DD carrier        c = dd + (b_k - b_ref) / lambda_k,  a = afv(c - (r_k - r_ref) / lambda_k)
@@ -32,6 +32,14 @@ struct ObsRow {
   double same;    // nonzero: the reference satellite is the previous row's
 };
 
+// The caller's rows as a kernel parameter: 32 of them are under the classic
+// 4 KB of parameters, sets above that take the larger one.
+constexpr int kObsRowsSmall = 32;
+template <int CAP>
+struct ObsRowsIn {
+  pf_obs_row_t row[CAP];
+};
+
 struct ObsBlock {
   int n;
   int kind;
@@ -42,6 +50,37 @@ struct ObsBlock {
   double gate;      // 0: no gate
   double huber_k;   // 0: Gaussian
 };
+
+// A row in the filter's local frame, every product and sum rounded by itself.
+template <int KIND>
+__device__ __forceinline__ ObsRow obs_row(const FilterDesc* fd, const FilterCtrl* fc, const pf_obs_row_t& r,
+                                          const pf_obs_row_t* prev) {
+  constexpr bool dd = KIND != PF_OBS_CARRIER_AFV;
+  ObsRow o;
+  double vk[3], vr[3];
+  for (int j = 0; j < 3; ++j) {
+    vk[j] = __dsub_rn(r.sat_k[j], fc->anchor[j]);
+    vr[j] = dd ? __dsub_rn(r.sat_ref[j], fc->anchor[j]) : 0.0;
+  }
+  for (int q = 0; q < 3; ++q) {
+    const double* m = fd->rot + 3 * q;
+    o.sk[q] = __dadd_rn(__dadd_rn(__dmul_rn(m[0], vk[0]), __dmul_rn(m[1], vk[1])), __dmul_rn(m[2], vk[2]));
+    o.sr[q] = __dadd_rn(__dadd_rn(__dmul_rn(m[0], vr[0]), __dmul_rn(m[1], vr[1])), __dmul_rn(m[2], vr[2]));
+  }
+  o.w = r.weight;
+  o.inv_wl = KIND == PF_OBS_DD_PSEUDORANGE ? 1.0 : 1.0 / r.wavelength;
+  if (KIND == PF_OBS_DD_PSEUDORANGE)
+    o.c = __dsub_rn(__dadd_rn(r.obs, r.base_k), r.base_ref);
+  else if (KIND == PF_OBS_CARRIER_AFV)
+    o.c = __dsub_rn(r.obs, __dmul_rn(fc->clk_anchor[0], o.inv_wl));
+  else
+    o.c = __dadd_rn(r.obs, __dmul_rn(__dsub_rn(r.base_k, r.base_ref), o.inv_wl));
+  o.same = dd && prev && prev->sat_ref[0] == r.sat_ref[0] && prev->sat_ref[1] == r.sat_ref[1] &&
+                   prev->sat_ref[2] == r.sat_ref[2]
+               ? 1.0
+               : 0.0;
+  return o;
+}
 
 // Residual of one row; rr holds the range to the previous row's reference
 // satellite (rows of a constellation share it), and this row's on return.
@@ -76,21 +115,15 @@ __device__ __forceinline__ double obs_cost(const ObsBlock& b, double w, double v
 // latter chooses one (the gate's test needed a pass of its own before, and every
 // row its own reference range).  FP64 roots bound it: 200K particles x 14
 // gated rows with two references, 36.4 -> 14.8 us.
-template <int KIND>
-__global__ void __launch_bounds__(kThreads) k_obs_term(EngineDev e, int f, ObsBlock b, const ObsRow* rows) {
-  __shared__ ObsRow s_rows[kMaxObsRows];
-  for (int i = threadIdx.x; i < b.n; i += kThreads) {
-    ObsRow r = rows[i];
-    r.same = 0.0;
-    if (i > 0) {
-      const ObsRow& q = rows[i - 1];
-      r.same = q.sr[0] == r.sr[0] && q.sr[1] == r.sr[1] && q.sr[2] == r.sr[2] ? 1.0 : 0.0;
-    }
-    s_rows[i] = r;
-  }
-  __syncthreads();
+template <int KIND, int CAP>
+__global__ void __launch_bounds__(kThreads) k_obs_term(EngineDev e, int f, ObsBlock b,
+                                                       const __grid_constant__ ObsRowsIn<CAP> in) {
+  __shared__ ObsRow s_rows[CAP];
   const FilterDesc* fd = e.desc + f;
   const FilterCtrl* fc = e.ctrl + f;
+  for (int i = threadIdx.x; i < b.n; i += kThreads)
+    s_rows[i] = obs_row<KIND>(fd, fc, in.row[i], i > 0 ? in.row + i - 1 : nullptr);
+  __syncthreads();
   const ParticleSrc ps = particle_src(e, fd, fc);
   const bool keep = b.accumulate && fc->lw_zero == 0;
   for (int j = blockIdx.x * kThreads + threadIdx.x; j < ps.n; j += gridDim.x * kThreads) {

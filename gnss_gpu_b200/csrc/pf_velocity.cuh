@@ -28,6 +28,10 @@ struct DopplerRow {
   double weight;
 };
 
+struct DopplerRowsIn {  // a call's rows, as a kernel parameter
+  DopplerRow row[kMaxDopplerRows];
+};
+
 // Two standard normals from two 32-bit words (Box-Muller in FP64).
 __device__ __forceinline__ void normals2_f64(uint32_t a, uint32_t b, double& z0, double& z1) {
   const double two_m32 = 2.3283064365386963e-10;
@@ -182,10 +186,12 @@ __global__ void __launch_bounds__(kThreads) k_vel_predict(EngineDev e, int f, co
   }
 }
 
-// The particles now sit, gathered, in the other state buffer.
-__global__ void k_flip_state(FilterCtrl* fc) {
+// The particles now sit, gathered, in the other state buffer; the error word goes
+// to its pinned mirror.
+__global__ void k_flip_state(FilterCtrl* fc, const unsigned* err, unsigned* err_map) {
   fc->parity ^= 1;
   fc->resample_flag = 0;
+  *err_map = *err;
 }
 
 // ECEF position of local offsets (x, y, z) about the filter's anchor.
@@ -238,11 +244,11 @@ __device__ __forceinline__ bool doppler_row(const DopplerSmem& r, const double (
 //    product of the mantissas plus the exponents.
 // Kernel time, 1M particles x 16 rows, WLS: 370 -> 72 us; 300K x 11, KF: 92 -> 43.
 template <bool KF>
-__global__ void __launch_bounds__(128) k_doppler(EngineDev e, int f, double* vb, const DopplerRow* rows,
-                                                DopplerArgs a) {
+__global__ void __launch_bounds__(128) k_doppler(EngineDev e, int f, double* vb,
+                                                const __grid_constant__ DopplerRowsIn in, DopplerArgs a) {
   __shared__ DopplerSmem s_rows[kMaxDopplerRows];
   for (int i = threadIdx.x; i < a.n_sat; i += blockDim.x) {
-    const DopplerRow r = rows[i];
+    const DopplerRow& r = in.row[i];
     DopplerSmem& o = s_rows[i];
     for (int k = 0; k < 3; ++k) {
       o.sat[k] = r.sat[k];
