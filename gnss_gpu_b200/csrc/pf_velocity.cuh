@@ -241,10 +241,16 @@ __device__ __forceinline__ bool doppler_row(const DopplerSmem& r, const double (
 //    whose unknown is the velocity, hence the right-hand side's 1e-9 terms).
 //  * KF: one reciprocal per row; the covariance is symmetric after the first
 //    update, so six elements are carried; sum log S as the logarithm of the
-//    product of the mantissas plus the exponents.
-// Kernel time, 1M particles x 16 rows, WLS: 370 -> 72 us; 300K x 11, KF: 92 -> 43.
+//    product of the mantissas plus the exponents.  A row that does not count
+//    is selected away instead of branched over, so that the next row's line of
+//    sight runs under the serial chain of this one (43 -> 38 us for 300K x 11;
+//    lines of sight kept in shared memory from the first pass: 51).
+// The chains are long, so warps matter more than registers: 6 CTAs per SM for KF
+// (5: 37.4 us, 4: 46, 6 with a few spilled words 36.1), 7 for WLS (the
+// compiler's choice: 80.6 us for 1M x 16, 6: 76.0, 7: 74.8, 8: 76.4).
+// Kernel time, 1M particles x 16 rows, WLS: 370 -> 72 us; 300K x 11, KF: 92 -> 36.
 template <bool KF>
-__global__ void __launch_bounds__(128) k_doppler(EngineDev e, int f, double* vb,
+__global__ void __launch_bounds__(128, KF ? 6 : 7) k_doppler(EngineDev e, int f, double* vb,
                                                 const __grid_constant__ DopplerRowsIn in, DopplerArgs a) {
   __shared__ DopplerSmem s_rows[kMaxDopplerRows];
   for (int i = threadIdx.x; i < a.n_sat; i += blockDim.x) {
@@ -350,17 +356,17 @@ __global__ void __launch_bounds__(128) k_doppler(EngineDev e, int f, double* vb,
         double P[9];
         for (int c = 0; c < 9; ++c) P[c] = vb[(size_t)(3 + c) * n + j];
         double pxx = P[0], pxy = P[1], pxz = P[2], pyy = P[4], pyz = P[5], pzz = P[8];
-        bool sym = P[1] == P[3] && P[2] == P[6] && P[5] == P[7];
+        const bool sym = P[1] == P[3] && P[2] == P[6] && P[5] == P[7];
         double quad = 0.0, mant = 1.0;
         int expo = 0;
         bool any = false;
-        for (int s = 0; s < a.n_sat; ++s) {
-          const DopplerSmem& r = s_rows[s];
+        auto row = [&](const DopplerSmem& r, auto symc) {
+          constexpr bool SYM = decltype(symc)::value;
           double l[3], y;
-          if (!(r.w > 0.0) || !doppler_row(r, pos, l, y)) continue;
+          const bool use = doppler_row(r, pos, l, y) && r.w > 0.0;
           const double h[3] = {-l[0] - hm[0], -l[1] - hm[1], -l[2] - hm[2]};
           double ph0, ph1, ph2, hp0, hp1, hp2;  // P h and h^T P
-          if (sym) {
+          if constexpr (SYM) {
             hp0 = ph0 = pxx * h[0] + pxy * h[1] + pxz * h[2];
             hp1 = ph1 = pxy * h[0] + pyy * h[1] + pyz * h[2];
             hp2 = ph2 = pxz * h[0] + pyz * h[1] + pzz * h[2];
@@ -373,39 +379,43 @@ __global__ void __launch_bounds__(128) k_doppler(EngineDev e, int f, double* vb,
             hp2 = h[0] * P[2] + h[1] * P[5] + h[2] * P[8];
           }
           const double S = h[0] * ph0 + h[1] * ph1 + h[2] * ph2 + r.var;
-          if (!(S > 1e-18) || !isfinite(S)) continue;
+          const bool good = use && S > 1e-18 && isfinite(S);
           const double iS = 1.0 / S;
           const double innov = (y - ym) - (h[0] * v[0] + h[1] * v[1] + h[2] * v[2]);
           const double k0 = ph0 * iS, k1 = ph1 * iS, k2 = ph2 * iS;
-          v[0] += k0 * innov;
-          v[1] += k1 * innov;
-          v[2] += k2 * innov;
-          if (!sym) {  // the first update leaves it symmetric
-            pxy = 0.5 * ((P[1] - k0 * hp1) + (P[3] - k1 * hp0));
-            pxz = 0.5 * ((P[2] - k0 * hp2) + (P[6] - k2 * hp0));
-            pyz = 0.5 * ((P[5] - k1 * hp2) + (P[7] - k2 * hp1));
-            sym = true;
+          const double v0 = v[0] + k0 * innov, v1 = v[1] + k1 * innov, v2 = v[2] + k2 * innov;
+          double nxy, nxz, nyz;
+          if constexpr (!SYM) {  // the first update leaves it symmetric
+            nxy = 0.5 * ((P[1] - k0 * hp1) + (P[3] - k1 * hp0));
+            nxz = 0.5 * ((P[2] - k0 * hp2) + (P[6] - k2 * hp0));
+            nyz = 0.5 * ((P[5] - k1 * hp2) + (P[7] - k2 * hp1));
           } else {
-            pxy -= k0 * hp1;
-            pxz -= k0 * hp2;
-            pyz -= k1 * hp2;
+            nxy = pxy - k0 * hp1;
+            nxz = pxz - k0 * hp2;
+            nyz = pyz - k1 * hp2;
           }
-          pxx -= k0 * hp0;
-          pyy -= k1 * hp1;
-          pzz -= k2 * hp2;
-          pxy = isfinite(pxy) ? pxy : 0.0;
-          pxz = isfinite(pxz) ? pxz : 0.0;
-          pyz = isfinite(pyz) ? pyz : 0.0;
-          pxx = (isfinite(pxx) && pxx > 1e-12) ? pxx : 1e-12;
-          pyy = (isfinite(pyy) && pyy > 1e-12) ? pyy : 1e-12;
-          pzz = (isfinite(pzz) && pzz > 1e-12) ? pzz : 1e-12;
-          any = true;
-          quad += innov * innov * iS;
+          const double nxx = pxx - k0 * hp0, nyy = pyy - k1 * hp1, nzz = pzz - k2 * hp2;
+          v[0] = good ? v0 : v[0];
+          v[1] = good ? v1 : v[1];
+          v[2] = good ? v2 : v[2];
+          pxy = good ? (isfinite(nxy) ? nxy : 0.0) : pxy;
+          pxz = good ? (isfinite(nxz) ? nxz : 0.0) : pxz;
+          pyz = good ? (isfinite(nyz) ? nyz : 0.0) : pyz;
+          pxx = good ? ((isfinite(nxx) && nxx > 1e-12) ? nxx : 1e-12) : pxx;
+          pyy = good ? ((isfinite(nyy) && nyy > 1e-12) ? nyy : 1e-12) : pyy;
+          pzz = good ? ((isfinite(nzz) && nzz > 1e-12) ? nzz : 1e-12) : pzz;
+          any |= good;
+          quad += good ? innov * innov * iS : 0.0;
           // S is a normal number above 1e-18: mantissa in [1, 2) and exponent
-          const long long bits = __double_as_longlong(S);
+          const long long bits = __double_as_longlong(good ? S : 1.0);
           expo += (int)(bits >> 52) - 1023;
           mant *= __longlong_as_double((bits & 0x000FFFFFFFFFFFFFll) | 0x3FF0000000000000ll);  // <= 2^64
-        }
+        };
+        int s = 0;
+        if (!sym)
+          while (s < a.n_sat && !any) row(s_rows[s++], std::false_type{});
+#pragma unroll 2
+        for (; s < a.n_sat; ++s) row(s_rows[s], std::true_type{});
         log_w = -0.5 * (quad + (log(mant) + (double)expo * 0.693147180559945309417));
         for (int i = 0; i < 3; ++i) vb[(size_t)i * n + j] = v[i];
         if (any) {
