@@ -1405,6 +1405,8 @@ int pfe_checkpoint_load(pf_engine_t* eng, int filter, const void* host_buf, size
   float* dst = c.parity ? eng->dev.state1 : eng->dev.state0;
   for (int dd = 0; dd < eng->D; ++dd) {
     CK(cudaMemcpy(dst + (size_t)dd * eng->P + base, in, sizeof(float) * n, cudaMemcpyHostToDevice));
+    if (n & 3)  // the rest of the last group (EngineDev::state0)
+      CK(cudaMemset(dst + (size_t)dd * eng->P + base + n, 0, sizeof(float) * (4 - (n & 3))));
     in += sizeof(float) * n;
   }
   CK(cudaMemcpy(eng->dev.lw + base, in, sizeof(float) * n, cudaMemcpyHostToDevice));

@@ -93,6 +93,9 @@ struct EngineDev {
   const FilterDesc* desc;
   FilterCtrl* ctrl;
   const int* tile_filter;
+  // The two state buffers.  Particles are read in groups of four, and a group's
+  // slots past the filter's end enter its sums with weight zero: whoever writes a
+  // filter's particles leaves finite values there too.
   float* state0;
   float* state1;
   float* lw;

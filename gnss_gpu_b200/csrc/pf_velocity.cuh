@@ -183,6 +183,9 @@ __global__ void __launch_bounds__(kThreads) k_vel_predict(EngineDev e, int f, co
       x[r] = (float)((double)x[r] + vp.rot[3 * r] * d[0] + vp.rot[3 * r + 1] * d[1] + vp.rot[3 * r + 2] * d[2]);
 #pragma unroll
     for (int d2 = 0; d2 < D; ++d2) dst[(size_t)d2 * e.p_total + j] = x[d2];
+    if (j == n - 1)  // fill the last group of four (EngineDev::state0)
+      for (int q = n; q & 3; ++q)
+        for (int d2 = 0; d2 < D; ++d2) dst[(size_t)d2 * e.p_total + q] = x[d2];
   }
 }
 
