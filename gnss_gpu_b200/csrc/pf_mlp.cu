@@ -49,6 +49,10 @@ struct GradSmem {
   float loss[kMlpThreads / 32];
 };
 
+// The kernels of a step start while their predecessor, which writes what they
+// read, still runs: their pointers are not __restrict__, so that no load may take
+// the read-only path, whose lines are not kept in step with other SMs' stores, or
+// move above the wait.
 __device__ __forceinline__ void mlp_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void mlp_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -89,8 +93,7 @@ __device__ __forceinline__ void b_frag_rows2(const __nv_bfloat16* src, int kt, i
 }
 
 __global__ void __launch_bounds__(kMlpThreads, 2)
-    k_mlp_grad(const float* __restrict__ X, const float* __restrict__ Y, int n, const float* __restrict__ prm,
-               float inv_n, float* __restrict__ partial) {
+    k_mlp_grad(const float* X, const float* Y, int n, const float* prm, float inv_n, float* partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(kMlpThreads, 2)
 // (m, v moments, step >= 1).  32 parameters per CTA, one group per warp.
 constexpr int kReduceGroups = 8;
 __global__ void __launch_bounds__(32 * kReduceGroups)
-    k_mlp_reduce(const float* __restrict__ partial, int nblk, float* grad, float* prm, float* m, float* v, int step,
+    k_mlp_reduce(const float* partial, int nblk, float* grad, float* prm, float* m, float* v, int step,
                  float lr, float inv_n, float* loss) {
   __shared__ float s_sum[kReduceGroups][32];
   mlp_pdl_trigger();

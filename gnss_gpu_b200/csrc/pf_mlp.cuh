@@ -81,7 +81,7 @@ struct MlpSmem {
 };
 
 // All threads of the CTA: FP32 master parameters -> BF16 shared copy.
-__device__ __forceinline__ void mlp_stage(const float* __restrict__ prm, MlpSmem& s, int nthreads) {
+__device__ __forceinline__ void mlp_stage(const float* prm, MlpSmem& s, int nthreads) {
   const uint2 zero = make_uint2(0u, 0u);
   auto four = [&](int off) {  // the parameter array is only known to be 4-byte aligned
     return make_uint2(pack_bf16(prm[off], prm[off + 1]), pack_bf16(prm[off + 2], prm[off + 3]));

@@ -308,7 +308,10 @@ constexpr int kTileS = 8;
 constexpr int kTileThreads = 32 * kTileS;
 
 // Programmatic dependent launch: the state table is needed by GLONASS tiles
-// only, so the orbit kernel starts while the table is made.
+// only, so the orbit kernel starts while the table is made.  What the previous
+// kernel writes (kmax, tbl) is not read through __restrict__ pointers: such a load
+// may take the read-only path, whose lines are not kept in step with other SMs'
+// stores, or move above the wait.
 __device__ inline void orbit_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ inline void orbit_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -353,7 +356,7 @@ __global__ void __launch_bounds__(kTileThreads) k_glo_need(const pf_broadcast_t*
 // The stored states: one thread per (record, direction) integrates kmax
 // full steps from toe and keeps every state (6 doubles each, kc per slot).
 __global__ void k_glo_table(const pf_broadcast_t* __restrict__ recs, int n_recs, double step,
-                            const int* __restrict__ kmax, int kc, double* __restrict__ tbl) {
+                            const int* kmax, int kc, double* __restrict__ tbl) {
   orbit_pdl_trigger();
   orbit_pdl_wait();  // kmax
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -384,7 +387,7 @@ __global__ void k_glo_table(const pf_broadcast_t* __restrict__ recs, int n_recs,
 template <int EPT>
 __global__ void __launch_bounds__(kTileThreads, 4) k_broadcast_orbits(const pf_broadcast_t* __restrict__ recs, int n_recs,
                                    const int* __restrict__ idx, const double* __restrict__ times,
-                                   int n_epoch, int n_sat, double glo_step, const double* __restrict__ tbl, int kc,
+                                   int n_epoch, int n_sat, double glo_step, const double* tbl, int kc,
                                    double* __restrict__ pos, double* __restrict__ clk, int* __restrict__ err) {
   constexpr int kE = 32 * EPT;
   __shared__ int s_idx[kE][kTileS + 1];
