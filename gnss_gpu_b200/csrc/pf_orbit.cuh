@@ -119,20 +119,34 @@ __device__ inline double recip(double x) {
 // one is below 1e-10: sine and cosine are then evaluated at E, and that last
 // update is applied to them (its square is below their rounding).  An update
 // needs no more than the leading digits of its divisor.
+//
+// Where that does not happen (e of about 0.98 and above, no broadcast orbit) the
+// updates wander, and the result is E after ten plain ones, stopping below 1e-15:
+// whatever E is, a point of the orbit.
 __device__ inline void kepler_solve(double M, double e, double& s, double& c) {
   double E = M;
   sincos(M, &s, &c);
   for (int k = 0; k < 10; ++k) {
     const double dE = (M - E + e * s) * recip<0>(1.0 - e * c);
     E += dE;
-    if (fabs(dE) < 1e-5) break;
+    if (fabs(dE) < 1e-5) {
+      sincos(E, &s, &c);
+      const double last = (M - E + e * s) * recip<0>(1.0 - e * c), s0 = s;
+      if (!(fabs(last) < 1e-5)) break;
+      s += c * last;
+      c -= s0 * last;
+      return;
+    }
     if (fabs(dE) <= kSmallAngle) rotate_small(s, c, dE);
     else sincos(E, &s, &c);
   }
+  E = M;
+  for (int k = 0; k < 10; ++k) {
+    const double dE = (M - E + e * sin(E)) / (1.0 - e * cos(E));
+    E += dE;
+    if (fabs(dE) < 1e-15) break;
+  }
   sincos(E, &s, &c);
-  const double dE = (M - E + e * s) * recip<0>(1.0 - e * c), s0 = s;
-  s += c * dE;
-  c -= s0 * dE;
 }
 
 // What a Kepler record's epochs share.
