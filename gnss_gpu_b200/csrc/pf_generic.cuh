@@ -17,8 +17,8 @@
 // GMM: c0 = log w_los - log sigma, c1 = -w / (2 sigma^2), c2, c3 the NLOS pair, -mu
 // in the place of mu; Huber: none; Student's t: c1 = w / (nu
 // sigma^2); Gaussian: c1 = -w / (2 sigma^2).  One likelihood holds for every
-// satellite, and one of weight <= 0 gets constants that add nothing, so the loops
-// are free of branches.
+// satellite, and one of weight <= 0 gets constants that add nothing and a finite
+// residual (its record may hold anything), so the loops are free of branches.
 #pragma once
 #include "pf_learned.cuh"
 
@@ -28,8 +28,8 @@ namespace pfb {
 __device__ __forceinline__ void write_generic_entry(float2* o, const EngineDev& e, float sigma, float eE, float eN,
                                                     float eU, float g, float y, float w) {
   const bool used = w > 0.f;
-  o[0] = bc(eE); o[1] = bc(eN); o[2] = bc(eU); o[3] = bc(0.5f * g);
-  o[4] = bc(y); o[5] = bc(used ? w : 0.f);
+  o[0] = bc(used ? eE : 0.f); o[1] = bc(used ? eN : 0.f); o[2] = bc(used ? eU : 0.f); o[3] = bc(used ? 0.5f * g : 0.f);
+  o[4] = bc(used ? y : 0.f); o[5] = bc(used ? w : 0.f);
   float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f, mu = 0.f;
   const float s2 = sigma * sigma;
   if (e.lk_type == PF_LIK_GMM) {
