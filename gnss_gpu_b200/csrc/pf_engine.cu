@@ -1731,6 +1731,12 @@ int pfe_vel_doppler(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const pf_d
   DopplerRowsIn in;
   memset(&in, 0, sizeof(in));
   memcpy(in.row, rows, sizeof(DopplerRow) * n_rows);
+  if (!kf) {  // the heaviest row first: the kernel takes its residuals from the first one (see there)
+    int top = 0;
+    for (int i = 1; i < n_rows; ++i)
+      if (rows[i].weight > rows[top].weight) top = i;
+    std::swap(in.row[0], in.row[top]);
+  }
   DopplerArgs a;
   memset(&a, 0, sizeof(a));
   a.n_sat = n_rows;

@@ -239,9 +239,14 @@ __device__ __forceinline__ bool doppler_row(const DopplerSmem& r, const double (
 //    implied clock drift at the particle's velocity, less that of the first
 //    row (so that nothing large is squared), the sums of w, w z, w z^2 give drift
 //    and likelihood, and the normal equations of z against (-l, 1) give the
-//    velocity correction itself; they are solved by LDL^T (the matrix is
-//    positive definite: 1e-9 is added to its diagonal, as in the reference,
-//    whose unknown is the velocity, hence the right-hand side's 1e-9 terms).
+//    velocity correction itself.  The host puts a row of the largest weight
+//    first: with z = 0 there, (sum w z)^2 / sum w is at most (1 - w0 / sum w)
+//    sum w z^2 (Cauchy and Schwarz), so the difference of the two keeps all but
+//    a factor of n rows, whatever the other rows hold (with a first row of weight
+//    0 and a Doppler of 1e6 Hz taken instead, log-weights were 8e-4 off).  The
+//    equations are solved by LDL^T (the matrix is positive definite: 1e-9 is
+//    added to its diagonal, as in the reference, whose unknown is the velocity,
+//    hence the right-hand side's 1e-9 terms).
 //  * KF: one reciprocal per row; the covariance is symmetric after the first
 //    update, so six elements are carried; sum log S as the logarithm of the
 //    product of the mantissas plus the exponents.  A row that does not count
