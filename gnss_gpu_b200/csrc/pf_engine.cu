@@ -1693,20 +1693,23 @@ int pfe_vel_predict(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const doub
   vp.kf = kf ? 1 : 0;
   vp.step = step;
   // a resample the velocity states have not followed yet is applied on the way
+  const bool follow = c.resample_flag && c.rs_seq != vs->seq;
+  const int sel = follow ? vs->sel ^ 1 : vs->sel;
   const double* vin = vs->buf + (size_t)vs->sel * kVelComp * d.n;
-  if (c.resample_flag && c.rs_seq != vs->seq) {
-    vs->sel ^= 1;
-    vs->seq = c.rs_seq;
-  }
-  double* vout = vs->buf + (size_t)vs->sel * kVelComp * d.n;
+  double* vout = vs->buf + (size_t)sel * kVelComp * d.n;
   switch (eng->D) {
     case 4: launch_vel_predict<4>(eng, filter, vin, vout, vp); break;
     case 5: launch_vel_predict<5>(eng, filter, vin, vout, vp); break;
     case 6: launch_vel_predict<6>(eng, filter, vin, vout, vp); break;
     default: launch_vel_predict<7>(eng, filter, vin, vout, vp); break;
   }
+  CK(cudaGetLastError());  // a refused launch leaves the filter and the velocity states as they were
   k_flip_state<<<1, 1, 0, eng->stream>>>(eng->ctrl_dev + filter, eng->dev.err, eng->err_host);
   CK(cudaGetLastError());
+  if (follow) {
+    vs->sel = sel;
+    vs->seq = c.rs_seq;
+  }
   c.parity ^= 1;
   c.resample_flag = 0;
   CK(cudaStreamSynchronize(eng->stream));

@@ -1,0 +1,118 @@
+"""Kernel launches that the driver refuses, made on the host: the library runs in a
+child process against a CUDA runtime without a GPU (tests/fake_cudart.c), which
+refuses the chosen call.  The library's call returns an error and leaves the
+filter as it was."""
+import json
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+HERE = Path(__file__).resolve().parent
+
+CHILD = r"""
+import ctypes as C, json, sys
+fake = C.CDLL(sys.argv[1], mode=C.RTLD_GLOBAL)
+fake.fake_log.restype = C.c_char_p
+sys.path.insert(0, sys.argv[2])
+import numpy as np
+from gnss_gpu_b200 import _native as N
+assert "torch" not in sys.modules   # it would bring the real runtime
+L = N.load()
+n, out = 4099, {}
+
+
+def launched(name):
+    return fake.fake_log().decode().count(name)
+
+
+def block(nbytes):   # 256-byte aligned memory
+    raw = C.create_string_buffer(nbytes + 256)
+    at = (C.addressof(raw) + 255) & ~255
+    keep.append(raw)
+    return C.c_void_p(at)
+
+
+keep = []
+cfg = N.EngineConfig(n_filters=1, n_clk=1, resampler=0, megopolis_iters=15, weight_mode=0, lw_mode=0, sys_offset=0,
+                     max_sats=16, obs_slots=1, flags=3, ess_threshold=0.5, huber_k=1.5)
+prm = (N.FilterParams * 1)()
+prm[0].n_particles, prm[0].seed, prm[0].sigma_clk, prm[0].sigma_pr = n, 3, 1.0, 3.0
+need, h, stream = C.c_size_t(0), C.c_void_p(), block(64)
+N.check(L.pfe_workspace_bytes(C.byref(cfg), prm, C.byref(need)))
+N.check(L.pfe_create(C.byref(cfg), prm, block(need.value), need, stream, C.byref(h)))
+p0, clk = np.array([-3957199.0, 3310205.0, 3737911.0]), np.zeros(4)
+N.check(L.pfe_initialize(h, 0, N.dptr(p0), N.dptr(clk), 5.0, 3.0))
+
+
+def control(**change):
+    # the five last words of the control block: rs_seq, resample_flag, lw_zero, parity, initialized
+    size = C.c_size_t(0)
+    N.check(L.pfe_checkpoint_bytes(h, 0, C.byref(size)))
+    blob = np.zeros(size.value, np.uint8)
+    N.check(L.pfe_checkpoint_save(h, 0, N.vptr(blob), size))
+    nctrl = int(blob[24:28].view(np.int32)[0])
+    words = blob[32 + 72:32 + 72 + nctrl].view(np.int32)
+    at = [i for i in range(len(words) - 4) if words[i + 4] == 1 and not words[i + 5:].any()][-1]
+    w = words[at:at + 5]
+    for k, v in change.items():
+        w[["rs_seq", "resample_flag", "lw_zero", "parity"].index(k)] = v
+    if change:
+        N.check(L.pfe_checkpoint_load(h, 0, N.vptr(blob), size))
+    return [int(x) for x in w]
+
+
+def refused(part, call):
+    fake.fake_clear_log()
+    fake.fake_refuse(part.encode())
+    status = call()
+    fake.fake_refuse(b"")
+    return status
+
+
+SCENARIO
+print(json.dumps(out))
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    d = tmp_path_factory.mktemp("fake_cudart")
+    so, ver = d / "libcudart.so.12", d / "version"
+    ver.write_text("libcudart.so.12 { global: *; };\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-Wl,-soname,libcudart.so.12", f"-Wl,--version-script={ver}",
+                    str(HERE / "fake_cudart.c"), "-o", str(so)], check=True)
+    return so
+
+
+def run(fake, scenario):
+    src = CHILD.replace("SCENARIO", scenario)
+    r = subprocess.run([sys.executable, "-c", src, str(fake), str(HERE.parent)], capture_output=True, text=True,
+                       timeout=120)
+    assert r.returncode == 0, r.stderr
+    return json.loads(r.stdout.splitlines()[-1])
+
+
+PREDICT = r"""
+vs = N.VelState()
+vs.buf = block(2 * 12 * n * 8)
+vs.sel, vs.seq = 0, 7
+out["control"] = control(resample_flag=1, rs_seq=9)
+g = np.zeros(3)
+predict = lambda: L.pfe_vel_predict(h, 0, C.byref(vs), N.dptr(g), 1.0, 0.5, 0.1, 0.5, 0, 0.0, 1)
+"""
+
+
+def test_velocity_predict_refused(fake):
+    """The filter keeps its buffer and its pending resample, the velocity state its
+    buffer; the next call follows the resample as if nothing had been."""
+    r = run(fake, PREDICT + r"""
+out["status"] = refused("k_vel_predict", predict)
+out["flips"], out["state"], out["after"] = launched("k_flip_state"), [vs.sel, vs.seq], control()
+out["again"] = predict()
+out["state_again"] = [vs.sel, vs.seq]
+""")
+    assert r["status"] != 0 and r["flips"] == 0
+    assert r["state"] == [0, 7] and r["after"] == r["control"]
+    assert r["again"] == 0 and r["state_again"] == [1, 9]
