@@ -1000,6 +1000,12 @@ int launch_weight_3d(pf_engine_t* eng, int filter, const MeshDev& m, const Sat3d
   memset(&cb, 0, sizeof(cb));
   unsigned char* buf = nullptr;
   RayMode mode = RAYS_WALK;
+  // each kernel reads what the one before it left: none follows a refused one
+  cudaError_t ce = cudaSuccess;
+  auto ok = [&] {
+    if (ce == cudaSuccess) ce = cudaGetLastError();
+    return ce == cudaSuccess;
+  };
   if (m.n_nodes > 0 && (long long)n * a.n_sat <= kThreadRays) {
     const size_t words = (size_t)(n + 31) / 32 * a.n_sat;
     if ((buf = (unsigned char*)scratch_alloc(sizeof(unsigned) * words, eng->stream))) {
@@ -1020,22 +1026,28 @@ int launch_weight_3d(pf_engine_t* eng, int filter, const MeshDev& m, const Sat3d
       cb.mark = (unsigned*)(buf + 1024);
       cb.code = (unsigned*)(buf + head);
       cb.list = (BlockList*)(buf + head + codes);
-      CK(cudaMemsetAsync(buf, 0, head, eng->stream));
-      k_cells_box<<<std::min(eng->sm_count * 2, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, cb.grid,
-                                                                                   a.n_sat);
-      k_cells_mark<<<std::min(eng->sm_count * 4, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, cb);
-      k_cells_block<<<(int)std::min<size_t>(eng->sm_count * 16, (blocks * a.n_sat + 127) / 128), 128, 0,
-                      eng->stream>>>(m, sv, a.n_sat, cb);
-      k_cells_cell<<<(int)std::min<size_t>(eng->sm_count * 8, (blocks * a.n_sat + 7) / 8), kThreads, 0,
-                     eng->stream>>>(m, sv, a.n_sat, cb);
+      ce = cudaMemsetAsync(buf, 0, head, eng->stream);
+      if (ok())
+        k_cells_box<<<std::min(eng->sm_count * 2, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, cb.grid,
+                                                                                     a.n_sat);
+      if (ok()) k_cells_mark<<<std::min(eng->sm_count * 4, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, cb);
+      if (ok())
+        k_cells_block<<<(int)std::min<size_t>(eng->sm_count * 16, (blocks * a.n_sat + 127) / 128), 128, 0,
+                        eng->stream>>>(m, sv, a.n_sat, cb);
+      if (ok())
+        k_cells_cell<<<(int)std::min<size_t>(eng->sm_count * 8, (blocks * a.n_sat + 7) / 8), kThreads, 0,
+                       eng->stream>>>(m, sv, a.n_sat, cb);
     }
   }
   const auto kernel = mode == RAYS_CELLS   ? k_weight_3d<RAYS_CELLS>
                       : mode == RAYS_WORDS ? k_weight_3d<RAYS_WORDS>
                                            : k_weight_3d<RAYS_WALK>;
-  kernel<<<std::min(eng->sm_count * 16, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a, cb);
-  CK(cudaGetLastError());
-  if (buf) CK(cudaFreeAsync(buf, eng->stream));
+  if (ok()) kernel<<<std::min(eng->sm_count * 16, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a, cb);
+  (void)ok();
+  const cudaError_t fe = buf ? cudaFreeAsync(buf, eng->stream) : cudaSuccess;
+  (void)cudaGetLastError();  // kept in ce and fe
+  CK(ce);
+  CK(fe);
   return PF_OK;
 }
 

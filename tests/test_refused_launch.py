@@ -20,7 +20,7 @@ import numpy as np
 from gnss_gpu_b200 import _native as N
 assert "torch" not in sys.modules   # it would bring the real runtime
 L = N.load()
-n, out = 4099, {}
+n, out = 40_003, {}
 
 
 def launched(name):
@@ -116,3 +116,37 @@ out["state_again"] = [vs.sel, vs.seq]
     assert r["status"] != 0 and r["flips"] == 0
     assert r["state"] == [0, 7] and r["after"] == r["control"]
     assert r["again"] == 0 and r["state_again"] == [1, 9]
+
+
+RAYS = r"""
+mesh = N.Mesh()
+mesh.nodes, mesh.tris, mesh.n_nodes, mesh.n_tris = block(64), block(64), 1, 1
+def term(n_sat):
+    sats = np.zeros(5 * n_sat)
+    return L.pfe_add_3d_term(h, 0, C.byref(mesh), N.dptr(sats), n_sat, 3.0, 30.0, 10.0, 0.8, 0.1, 0)
+out["base"], out["lw_zero"] = fake.fake_pool_blocks(), control()[2]
+N.check(term(1)); out["words"] = launched("k_rays_3d")
+N.check(term(64)); out["cells"] = launched("k_cells_cell")
+out["ok"] = fake.fake_pool_blocks()
+"""
+
+
+@pytest.mark.parametrize("n_sat,part", [(1, "k_rays_3d"), (1, "k_weight_3d"), (64, "k_cells_box"), (64, "k_cells_mark"),
+                                        (64, "k_cells_block"), (64, "k_cells_cell"), (64, "k_weight_3d"), (64, "fill")])
+def test_ray_scratch_goes_back_when_a_kernel_is_refused(fake, n_sat, part):
+    r = run(fake, RAYS + f"""
+fake.fake_refuse_fill(int("{part}" == "fill"))
+out["status"] = [refused("{part}" if "{part}" != "fill" else "", lambda: term({n_sat})) for _ in range(3)]
+fake.fake_refuse_fill(0)
+out["done"] = launched("k_term_done")
+out["later"] = fake.fake_log().decode().splitlines()
+out["after"] = fake.fake_pool_blocks()
+out["again"] = term({n_sat})
+""")
+    assert r["words"] == 1 and r["cells"] == 1 and r["ok"] == r["base"]  # both routes were taken
+    assert all(r["status"]) and r["done"] == 0 and r["again"] == 0
+    assert r["after"] == r["base"]
+    chain = ["k_rays_3d", "k_weight_3d"] if n_sat == 1 else ["k_cells_box", "k_cells_mark", "k_cells_block",
+                                                              "k_cells_cell", "k_weight_3d"]
+    before = chain[:chain.index(part)] if part != "fill" else []
+    assert len(r["later"]) == len(before) and all(b in ln for b, ln in zip(before, r["later"]))
