@@ -1613,6 +1613,7 @@ int pfe_add_obs_term(pf_engine_t* eng, int filter, int kind, const pf_obs_row_t*
     case PF_OBS_CARRIER_AFV: launch_obs_term<PF_OBS_CARRIER_AFV>(eng, filter, b, rows); break;
     default: launch_obs_term<PF_OBS_DD_CARRIER_AFV>(eng, filter, b, rows); break;
   }
+  CK(cudaGetLastError());
   return term_done(eng, filter);
 }
 

@@ -150,3 +150,18 @@ out["again"] = term({n_sat})
                                                               "k_cells_cell", "k_weight_3d"]
     before = chain[:chain.index(part)] if part != "fill" else []
     assert len(r["later"]) == len(before) and all(b in ln for b, ln in zip(before, r["later"]))
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("rows", [4, 40])
+def test_observation_term_refused(fake, kind, rows):
+    """The log-weights stay read as zero, as before the call."""
+    r = run(fake, f"""
+rows = np.zeros({rows}, N.OBS_ROW_DTYPE)
+rows["weight"], rows["wavelength"] = 1.0, 0.19
+term = lambda: L.pfe_add_obs_term(h, 0, {kind}, N.vptr(rows), {rows}, 1.0, 0.0, 0.0, 0)
+out["status"], out["done"], out["again"] = refused("k_obs_term", term), launched("k_term_done"), term()
+out["done_again"] = launched("k_term_done")
+""")
+    assert r["status"] != 0 and r["done"] == 0
+    assert r["again"] == 0 and r["done_again"] == 1
