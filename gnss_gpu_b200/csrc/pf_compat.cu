@@ -778,24 +778,28 @@ int pf_broadcast_orbits(const pf_broadcast_t* d_recs, int n_recs, const int* d_r
   if (ce == cudaSuccess) {
     k_glo_need<<<(unsigned)(st_tiles * ((n_epoch + kNeedE - 1) / kNeedE)), kTileThreads, 0, st>>>(
         d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step, kc, kmax);
-    cudaLaunchConfig_t lc;
-    memset(&lc, 0, sizeof(lc));
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    lc.stream = st;
+    ce = cudaGetLastError();
+  }
+  cudaLaunchConfig_t lc;
+  memset(&lc, 0, sizeof(lc));
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  lc.stream = st;
+  if (ce == cudaSuccess) {
     lc.gridDim = dim3((unsigned)((2 * n_recs + 31) / 32));  // a serial walk per thread: one warp per CTA
     lc.blockDim = dim3(32);
     ce = cudaLaunchKernelEx(&lc, k_glo_table, d_recs, n_recs, glo_step, (const int*)kmax, kc, tbl);
-    if (ce == cudaSuccess) {
-      lc.gridDim = dim3(grid);
-      lc.blockDim = dim3(kTileThreads);
-      ce = cudaLaunchKernelEx(&lc, orbits, d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step,
-                              (const double*)tbl, kc, d_pos, d_clk, (int*)nullptr);
-    }
   }
+  if (ce == cudaSuccess) {
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(kTileThreads);
+    ce = cudaLaunchKernelEx(&lc, orbits, d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step,
+                            (const double*)tbl, kc, d_pos, d_clk, (int*)nullptr);
+  }
+  (void)cudaGetLastError();  // kept in ce
   const cudaError_t fe = cudaFreeAsync(scratch, st);
   CK(ce);
   CK(fe);

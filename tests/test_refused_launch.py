@@ -165,3 +165,25 @@ out["done_again"] = launched("k_term_done")
 """)
     assert r["status"] != 0 and r["done"] == 0
     assert r["again"] == 0 and r["done_again"] == 1
+
+
+@pytest.mark.parametrize("part", ["k_glo_need", "k_glo_table", "k_broadcast_orbits", "fill"])
+def test_orbits_refused(fake, part):
+    """No later kernel runs on a table that was not made, and the scratch goes back."""
+    r = run(fake, f"""
+rec = np.zeros(4, N.BROADCAST_DTYPE)
+rec["system"] = ord("R")
+t, pos, clk = np.arange(100.0), np.zeros((100, 4, 3)), np.zeros((100, 4))
+orbits = lambda: L.pf_broadcast_orbits(N.vptr(rec), 4, None, N.vptr(t), 100, 4, 60.0, N.vptr(pos), N.vptr(clk), None)
+N.check(orbits())
+out["chain"], out["base"] = fake.fake_log().decode().splitlines()[-3:], fake.fake_pool_blocks()
+fake.fake_refuse_fill(int("{part}" == "fill"))
+out["status"] = refused("{part}" if "{part}" != "fill" else "", orbits)
+fake.fake_refuse_fill(0)
+out["ran"], out["after"], out["again"] = fake.fake_log().decode().splitlines(), fake.fake_pool_blocks(), orbits()
+""")
+    names = ["k_glo_need", "k_glo_table", "k_broadcast_orbits"]
+    assert len(r["chain"]) == 3 and all(n in ln for n, ln in zip(names, r["chain"]))
+    before = names[:names.index(part)] if part != "fill" else []
+    assert r["status"] != 0 and len(r["ran"]) == len(before)
+    assert r["after"] == r["base"] and r["again"] == 0
