@@ -432,8 +432,8 @@ int read_ctrl(pf_engine* eng) {
 // The end of a call that wrote log-weights of filter f: the weights are explicit
 // now, and the error word goes to its pinned mirror.  One thread does both in one
 // launch (a 4-byte copy in each direction took its place before).
-int term_done(pf_engine* eng, int f) {
-  k_term_done<<<1, 1, 0, eng->stream>>>(eng->ctrl_dev + f, eng->dev.err, eng->err_host);
+int term_done(pf_engine* eng, int f, bool if_clean = false) {
+  k_term_done<<<1, 1, 0, eng->stream>>>(eng->ctrl_dev + f, eng->dev.err, eng->err_host, if_clean);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(eng->stream));
   return err_status(*eng->err_host);
@@ -1614,7 +1614,7 @@ int pfe_add_obs_term(pf_engine_t* eng, int filter, int kind, const pf_obs_row_t*
     default: launch_obs_term<PF_OBS_DD_CARRIER_AFV>(eng, filter, b, rows); break;
   }
   CK(cudaGetLastError());
-  return term_done(eng, filter);
+  return term_done(eng, filter, true);  // the kernel leaves the weights of a filter in error
 }
 
 static int vel_check(pf_engine_t* eng, int filter, pf_vel_state_t* vs) {

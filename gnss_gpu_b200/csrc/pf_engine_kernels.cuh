@@ -1533,11 +1533,12 @@ __global__ void __launch_bounds__(kThreads) k_position_term(EngineDev e, int f, 
   }
 }
 
-// The end of a call that wrote log-weights: they are explicit now, and the error
-// word goes to its pinned mirror.
-__global__ void k_term_done(FilterCtrl* fc, const unsigned* err, unsigned* err_map) {
-  fc->lw_zero = 0;
-  *err_map = *err;
+// The end of a call that wrote log-weights: they are explicit now (if_clean: unless
+// an error was set), and the error word goes to its pinned mirror.
+__global__ void k_term_done(FilterCtrl* fc, const unsigned* err, unsigned* err_map, bool if_clean) {
+  const unsigned w = *err;
+  if (!if_clean || w == 0u) fc->lw_zero = 0;
+  *err_map = w;
 }
 
 // Control blocks and error word to their pinned mirror (words of 4 bytes).

@@ -119,6 +119,7 @@ template <int KIND, int CAP>
 __global__ void __launch_bounds__(kThreads) k_obs_term(EngineDev e, int f, ObsBlock b,
                                                        const __grid_constant__ ObsRowsIn<CAP> in) {
   __shared__ ObsRow s_rows[CAP];
+  if (__ldcg(e.err)) return;  // an earlier step's error: reported by the call, the weights stay
   const FilterDesc* fd = e.desc + f;
   const FilterCtrl* fc = e.ctrl + f;
   for (int i = threadIdx.x; i < b.n; i += kThreads)
