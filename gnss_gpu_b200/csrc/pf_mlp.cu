@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_forward(const float* __rest
 }
 
 constexpr int kGradBlocks = 296;  // two CTAs per SM
+constexpr int kMinPartials = 64;  // partial gradients that a caller's scratch must hold at least
 
 // Launch that may start while the stream's previous kernel drains (the kernel
 // waits for its results with griddepcontrol.wait).
@@ -379,9 +380,13 @@ int pf_mlp_param_count(void) { return kMlpParams; }
 
 size_t pf_mlp_scratch_bytes(void) { return (size_t)kGradBlocks * kMlpPart * sizeof(float); }
 
+// On as many CTAs as the rows fill, the SMs hold and the scratch has room for
+// (gradient of 100,000 rows: 32 us with room for 296, 84 with 64).
 static int grad_launch(const float* d_x, const float* d_y, int n, const float* d_params, float* d_scratch,
-                       int* nblk_out, cudaStream_t st) {
-  const int nblk = std::min(kGradBlocks, (n + kRows - 1) / kRows);
+                       size_t scratch_bytes, int* nblk_out, cudaStream_t st) {
+  const size_t room = scratch_bytes / (kMlpPart * sizeof(float));
+  if (room < (size_t)kMinPartials) return set_err(PF_EINVAL, "scratch too small");
+  const int nblk = (int)std::min({(size_t)kGradBlocks, ((size_t)n + kRows - 1) / kRows, room});
   const size_t smem = sizeof(GradSmem);
   cudaError_t e = cudaFuncSetAttribute((const void*)k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return set_err(PF_ECUDA, "mlp grad attribute: %s", cudaGetErrorString(e));
@@ -396,10 +401,9 @@ int pf_mlp_grad(const float* d_x, const float* d_y, int n, const float* d_params
   clear_err();
   if (!d_x || !d_y || !d_params || !d_grad || !d_scratch) return set_err(PF_EINVAL, "null pointer");
   if (n <= 0) return set_err(PF_EINVAL, "n must be > 0");
-  if (scratch_bytes < pf_mlp_scratch_bytes()) return set_err(PF_EINVAL, "scratch too small");
   cudaStream_t st = (cudaStream_t)stream;
   int nblk = 0, s;
-  if ((s = grad_launch(d_x, d_y, n, d_params, (float*)d_scratch, &nblk, st)) != PF_OK) return s;
+  if ((s = grad_launch(d_x, d_y, n, d_params, (float*)d_scratch, scratch_bytes, &nblk, st)) != PF_OK) return s;
   cudaError_t e = launch_pdl(k_mlp_reduce, (kMlpParams + 32) / 32, 32 * kReduceGroups, 0, st, (const float*)d_scratch,
                              nblk, d_grad, (float*)nullptr, (float*)nullptr, (float*)nullptr, 0, 0.f,
                              1.0f / (float)n, d_loss);
@@ -411,10 +415,9 @@ int pf_mlp_adam_step(const float* d_x, const float* d_y, int n, float* d_params,
   clear_err();
   if (!d_x || !d_y || !d_params || !d_m || !d_v || !d_scratch) return set_err(PF_EINVAL, "null pointer");
   if (n <= 0 || step < 1 || !(lr > 0.f)) return set_err(PF_EINVAL, "bad n, step or lr");
-  if (scratch_bytes < pf_mlp_scratch_bytes()) return set_err(PF_EINVAL, "scratch too small");
   cudaStream_t st = (cudaStream_t)stream;
   int nblk = 0, s;
-  if ((s = grad_launch(d_x, d_y, n, d_params, (float*)d_scratch, &nblk, st)) != PF_OK) return s;
+  if ((s = grad_launch(d_x, d_y, n, d_params, (float*)d_scratch, scratch_bytes, &nblk, st)) != PF_OK) return s;
   cudaError_t e = launch_pdl(k_mlp_reduce, (kMlpParams + 32) / 32, 32 * kReduceGroups, 0, st, (const float*)d_scratch,
                              nblk, (float*)nullptr, d_params, d_m, d_v, step, lr, 1.0f / (float)n, d_loss);
   return e == cudaSuccess ? PF_OK : set_err(PF_ECUDA, "mlp adam: %s", cudaGetErrorString(e));

@@ -564,6 +564,8 @@ int pfe_get_sat_debug(pf_engine_t* eng, int filter, float* out, int max_sats, in
  * `stream`.  Loss: mean over rows of BCE(p, nlos) + nlos ((mu - bias)/20)^2.
  */
 int pf_mlp_param_count(void);
+/* Scratch for the two calls below at full speed.  They take less, down to 64
+ * partial gradients of (param_count + 1) floats, and then run on fewer CTAs. */
 size_t pf_mlp_scratch_bytes(void);
 /* Gradient of the mean loss (d_grad, param_count floats) and the loss. */
 int pf_mlp_grad(const float* d_x, const float* d_y, int n, const float* d_params,
