@@ -992,7 +992,8 @@ namespace {
 // The 3D likelihood of one filter: a thread per ray, per particle, or the
 // shadow cells of the cloud (the rule's reasons are at kThreadRays).  The scratch
 // (at most 34 MB) comes from the library's stream-ordered pool and goes back to
-// it within the call; without it every particle's thread walks its own rays.
+// it within the call; without it, or for a cloud too wide for cells (kCellSpan),
+// every particle's thread walks its own rays.
 int launch_weight_3d(pf_engine_t* eng, int filter, const MeshDev& m, const Sat3d* sv, const Weight3dArgs& a) {
   const int n = eng->hdesc[filter].n;
   const int tiles = (n + kThreads - 1) / kThreads;
@@ -1028,7 +1029,7 @@ int launch_weight_3d(pf_engine_t* eng, int filter, const MeshDev& m, const Sat3d
       cb.list = (BlockList*)(buf + head + codes);
       ce = cudaMemsetAsync(buf, 0, head, eng->stream);
       if (ok())
-        k_cells_box<<<std::min(eng->sm_count * 2, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, cb.grid,
+        k_cells_box<<<std::min(kBoxSample / kThreads, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, cb.grid,
                                                                                      a.n_sat);
       if (ok()) k_cells_mark<<<std::min(eng->sm_count * 4, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, cb);
       if (ok())
@@ -1039,10 +1040,14 @@ int launch_weight_3d(pf_engine_t* eng, int filter, const MeshDev& m, const Sat3d
                        eng->stream>>>(m, sv, a.n_sat, cb);
     }
   }
-  const auto kernel = mode == RAYS_CELLS   ? k_weight_3d<RAYS_CELLS>
-                      : mode == RAYS_WORDS ? k_weight_3d<RAYS_WORDS>
-                                           : k_weight_3d<RAYS_WALK>;
-  if (ok()) kernel<<<std::min(eng->sm_count * 16, tiles), kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a, cb);
+  const int g = std::min(eng->sm_count * 16, tiles);
+  if (mode == RAYS_WORDS) {
+    if (ok()) k_weight_3d<RAYS_WORDS><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a, cb);
+  } else {
+    if (ok() && mode == RAYS_CELLS)
+      k_weight_3d<RAYS_CELLS><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a, cb);
+    if (ok()) k_weight_3d<RAYS_WALK><<<g, kThreads, 0, eng->stream>>>(eng->dev, filter, m, sv, a, cb);
+  }
   (void)ok();
   const cudaError_t fe = buf ? cudaFreeAsync(buf, eng->stream) : cudaSuccess;
   (void)cudaGetLastError();  // kept in ce and fe

@@ -16,7 +16,8 @@ namespace pfb {
 // nearly the same question a million times: the cloud is a few metres wide.
 // So the cloud's box is cut into cells and these into blocks of 4 x 4 x 2, and
 // the rays from a block (a cell) to a satellite are treated as one beam:
-//   k_cells_box     mean and spread of the particles' offsets -> the grid
+//   k_cells_box     mean and spread of the particles' offsets -> the grid, or none
+//                   for a cloud too wide for cells (kCellSpan)
 //   k_cells_mark    which blocks hold particles
 //   k_cells_block   per (block, satellite) one walk of the hierarchy with the
 //                   beam's centre ray and boxes enlarged by its half extents;
@@ -47,6 +48,7 @@ constexpr unsigned kCodePerRay = 1u << 30;    // or one of these
 constexpr int kBlockCells = 32;               // 4 x 4 x 2
 constexpr int kCellsMax = 1 << 18;            // cells of a grid
 constexpr int kCellItems = 1 << 22;           // cells x satellites
+constexpr int kBoxSample = 1 << 16;           // particles that place the grid
 // Rays (particles x satellites) up to which each gets its own thread, and above
 // which the cells pay.  Likelihood alone, us, one thread per particle / this
 // rule: 3,000 x 16 95 / 42, 10,000 x 24 132 / 53, 60,000 x 16 132 / 122, 180,000 x
@@ -54,6 +56,17 @@ constexpr int kCellItems = 1 << 22;           // cells x satellites
 // cloud the more); 200,000 x 10, 125 / 140 with cells, hence the line above it.
 constexpr long long kThreadRays = 1000000;
 constexpr long long kCellRays = 2200000;
+// Cells wider than this share of the spacing of the mesh's triangles settle too
+// little: most lists overflow or hold many triangles per ray, and every particle
+// walks its own rays instead (n_blocks = 0).  The cloud's width is known on the
+// device only, so both kernels are launched and one returns at once.  Likelihood
+// alone, us, walks / cells: city of 2,490 triangles at 40 m spacing, 1M x 16
+// particles spread by 50, 100, 140, 200, 300 m (cells of 0.18, 0.36, 0.50, 0.72,
+// 1.07 spacings) 1213 / 614, 1285 / 923, 1263 / 1103, 1233 / 2333, 1187 / 2975; the
+// same triangles in four, 1M, 0.36 and 0.50 spacings 1559 / 1006, 1591 / 1967; 200K x
+// 16, 0.28 and 0.55 spacings 328 / 246, 351 / 352.  A cloud sent back costs some 20 us
+// over the walks (300 m: 1206 us, 150K x 16 particles 263 against 241).
+constexpr float kCellSpan = 0.45f;
 #ifndef PF_CELL_PARTICLES
 #define PF_CELL_PARTICLES 8
 #endif
@@ -71,7 +84,7 @@ struct CellGrid {
   float lo[3];
   float side, inv_side;
   int bdim[3];   // blocks
-  int n_blocks;
+  int n_blocks;  // 0: no cells, the particles walk
   float M[9];    // local offsets -> mesh frame: M x + off
   float off[3];
   float hm[3];   // |M| (1, 1, 1)
@@ -260,9 +273,24 @@ __device__ __forceinline__ void beam_walk(const MeshDev& m, const float3 c, cons
   out->n = kCodePerRay;
 }
 
-// Mean and spread of the offsets (exact integer sums, so the grid does not
-// depend on the order), then the grid: cubic cells over the mean +- 4.2
-// standard deviations (outside it rays walk by themselves, 30 times the work),
+// Mean horizontal spacing of the mesh's triangles: the square root of its area
+// over their number.
+__device__ __forceinline__ float tri_spacing(const MeshDev& m) {
+  float lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY};
+  for (int k = 0; k < 2; ++k) {  // the root's children (an unused one is at 1e30)
+    const float4 mn = __ldg(m.nodes + 2 * k), mx = __ldg(m.nodes + 2 * k + 1);
+    if (mn.x >= 1e29f) continue;
+    lo[0] = fminf(lo[0], mn.x);
+    lo[1] = fminf(lo[1], mn.y);
+    hi[0] = fmaxf(hi[0], mx.x);
+    hi[1] = fmaxf(hi[1], mx.y);
+  }
+  return sqrtf((hi[0] - lo[0]) * (hi[1] - lo[1]) / (float)m.n_tris);
+}
+
+// Mean and spread of the offsets of about kBoxSample particles (exact integer sums,
+// so the grid does not depend on the order), then the grid: cubic cells over the
+// mean +- 4.2 standard deviations (outside it rays walk by themselves, 30 times the work),
 // about n / PF_CELL_PARTICLES within +- 3.2.
 __global__ void __launch_bounds__(kThreads) k_cells_box(EngineDev e, int f, MeshDev m, CellGrid* g, int n_sat) {
   const FilterDesc* fd = e.desc + f;
@@ -270,8 +298,11 @@ __global__ void __launch_bounds__(kThreads) k_cells_box(EngineDev e, int f, Mesh
   const ParticleSrc ps = particle_src(e, fd, fc);
   long long s1[3] = {0, 0, 0}, s2[3] = {0, 0, 0};
   unsigned cnt = 0;
-  for (int j = blockIdx.x * kThreads + threadIdx.x; j < ps.n; j += gridDim.x * kThreads) {
-    const float* sp = particle_at(e, ps, j);
+  const int step = max(1, ps.n / kBoxSample);  // of warps
+  for (int i = blockIdx.x * kThreads + threadIdx.x;; i += gridDim.x * kThreads) {
+    const long long j = (long long)(i >> 5) * step * 32 + (i & 31);
+    if (j >= ps.n) break;
+    const float* sp = particle_at(e, ps, (int)j);
     const float x[3] = {__ldcg(sp), __ldcg(sp + e.p_total), __ldcg(sp + 2 * e.p_total)};
     if (!(isfinite(x[0]) && isfinite(x[1]) && isfinite(x[2]))) continue;
     ++cnt;
@@ -343,7 +374,7 @@ __global__ void __launch_bounds__(kThreads) k_cells_box(EngineDev e, int f, Mesh
   }
   g->side = side;
   g->inv_side = 1.0f / side;
-  g->n_blocks = dim[0] * dim[1] * dim[2];
+  g->n_blocks = side <= kCellSpan * tri_spacing(m) ? dim[0] * dim[1] * dim[2] : 0;
   const double* rf = fd->rot;
   for (int r = 0; r < 3; ++r) {
     double o = 0.0;
@@ -381,6 +412,7 @@ __global__ void __launch_bounds__(kThreads) k_cells_mark(EngineDev e, int f, Cel
   __shared__ unsigned s_bits[kCellsMax / kBlockCells / 32 + 1];  // marks collected per CTA: few words, many writers
   const ParticleSrc ps = particle_src(e, e.desc + f, e.ctrl + f);
   const int words = (cb.grid->n_blocks + 31) / 32;
+  if (words == 0) return;
   for (int i = threadIdx.x; i < words; i += kThreads) s_bits[i] = 0u;
   __syncthreads();
   for (int j = blockIdx.x * kThreads + threadIdx.x; j < ps.n; j += gridDim.x * kThreads) {
@@ -477,6 +509,9 @@ __global__ void __launch_bounds__(kThreads, MODE == RAYS_CELLS ? 3 : 4) k_weight
                                                                                    CellBufs cb) {
   constexpr int kWarps = kThreads / 32, kQueue = 64;
   constexpr int kSlots = MODE == RAYS_CELLS ? kWarps : 1;  // the queues are the cells'
+  // with a grid, its kernel and the walking one are both launched: the cloud decides
+  if (MODE == RAYS_CELLS && cb.grid->n_blocks == 0) return;
+  if (MODE == RAYS_WALK && cb.grid && cb.grid->n_blocks != 0) return;
   __shared__ Sat3d s_sat[kMax3dSats];
   __shared__ double s_p[kSlots][3][32];
   __shared__ unsigned long long s_blk[kSlots][32];

@@ -147,7 +147,7 @@ out["again"] = term({n_sat})
     assert all(r["status"]) and r["done"] == 0 and r["again"] == 0
     assert r["after"] == r["base"]
     chain = ["k_rays_3d", "k_weight_3d"] if n_sat == 1 else ["k_cells_box", "k_cells_mark", "k_cells_block",
-                                                              "k_cells_cell", "k_weight_3d"]
+                                                              "k_cells_cell", "k_weight_3d", "k_weight_3d"]
     before = chain[:chain.index(part)] if part != "fill" else []
     assert len(r["later"]) == len(before) and all(b in ln for b, ln in zip(before, r["later"]))
 
