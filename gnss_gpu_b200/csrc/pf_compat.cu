@@ -746,11 +746,19 @@ int pf_broadcast_orbits(const pf_broadcast_t* d_recs, int n_recs, const int* d_r
   if (!isfinite(glo_step) || glo_step <= 0.0) glo_step = kGloStep;
   if (glo_step < 1.0) return set_err(PF_EINVAL, "glo_step below 1 s");
   cudaStream_t st = (cudaStream_t)stream;
-  const long st_tiles = (n_sat + kTileS - 1) / kTileS, need_tiles = st_tiles * ((n_epoch + 31) / 32);
-  // four epochs per thread once that still gives every SM its CTAs
-  const bool four = need_tiles >= 4 * 148 * 4;
-  const unsigned grid = (unsigned)(st_tiles * ((n_epoch + (four ? 127 : 31)) / (four ? 128 : 32)));
-  const auto orbits = four ? k_broadcast_orbits<4> : k_broadcast_orbits<1>;
+  int dev = 0, sms = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // tiles of one satellite or of eight (kNarrowSats), of four epochs per thread
+  // once that still gives every SM its four CTAs
+  const bool narrow = n_sat <= kNarrowSats;
+  const int ts = narrow ? 1 : kTileS, rows = 32 * kTileS / ts;
+  const long cols = (n_sat + ts - 1) / ts, tiles = cols * (((long)n_epoch + rows - 1) / rows);
+  const bool four = tiles >= 4l * sms * 4;
+  const unsigned grid = (unsigned)(four ? cols * (((long)n_epoch + 4 * rows - 1) / (4 * rows)) : tiles);
+  const auto orbits = narrow ? (four ? k_broadcast_orbits<4, 1> : k_broadcast_orbits<1, 1>)
+                             : (four ? k_broadcast_orbits<4, kTileS> : k_broadcast_orbits<1, kTileS>);
+  const long need_cols = (n_sat + kTileS - 1) / kTileS;
   // GLONASS state table: the epochs of a record share its states at whole
   // steps from toe, so they are integrated once per (record, direction)
   int kc = 0;
@@ -776,7 +784,7 @@ int pf_broadcast_orbits(const pf_broadcast_t* d_recs, int n_recs, const int* d_r
   double* tbl = (double*)(scratch + kmax_bytes);
   cudaError_t ce = cudaMemsetAsync(kmax, 0, kmax_bytes, st);
   if (ce == cudaSuccess) {
-    k_glo_need<<<(unsigned)(st_tiles * ((n_epoch + kNeedE - 1) / kNeedE)), kTileThreads, 0, st>>>(
+    k_glo_need<<<(unsigned)(need_cols * (((long)n_epoch + kNeedE - 1) / kNeedE)), kTileThreads, 0, st>>>(
         d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step, kc, kmax);
     ce = cudaGetLastError();
   }

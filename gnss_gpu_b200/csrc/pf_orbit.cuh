@@ -314,12 +314,21 @@ __device__ inline int orbit_record(const int* idx, long i, int s, int n_recs) {
   return (r < 0 || r >= n_recs) ? -1 : r;
 }
 
-// Tiles of kTileE epochs x 8 satellites per CTA: a warp takes epochs of one
+// Tiles of 32 EPT epochs x 8 satellites per CTA: a warp takes epochs of one
 // satellite, so its lanes run the same orbit model with similar step counts, and
 // the CTA's eight satellites make the row-major arrays' segments (8 indexes, 8
 // positions, 8 clocks of an epoch) whole sectors.
 constexpr int kTileS = 8;
 constexpr int kTileThreads = 32 * kTileS;
+// Up to this many satellites a tile is 256 EPT epochs x 1 satellite: the warps of
+// the missing satellites would only wait.  Whole calls, us, tiles of eight / of one
+// (and one thread per satellite-epoch, before the tiles): Kepler 1 x 1M epochs 194 /
+// 55 (71), 2 x 500K 112 / 56 (69), 4 x 86,400 40 / 26 (37), GLONASS 1 x 1M 221 / 120
+// (201), 4 x 86,400 207 / 114 (308); 1 to 4 x 100 to 3,000 equal.  From five on the
+// tiles of eight are ahead of the thread per satellite-epoch (5 x 86,400 42 (43), 7 x
+// 86,400 46 (53)) and of the other tile where GLONASS rows are short (7 x 20,000 109
+// / 141).
+constexpr int kNarrowSats = 4;
 
 // Programmatic dependent launch: the state table is needed by GLONASS tiles
 // only, so the orbit kernel starts while the table is made.  What the previous
@@ -395,36 +404,36 @@ __global__ void k_glo_table(const pf_broadcast_t* __restrict__ recs, int n_recs,
 // FP64 bound (36 bytes a satellite-epoch are 31 us of the day-long call at
 // the measured copy rate).  Each thread takes EPT epochs of its satellite and
 // keeps what its record's epochs share; results go through shared memory, so
-// that positions and clocks leave as whole rows of eight satellites.  A day at
+// that positions and clocks leave as whole rows of TS satellites.  A day at
 // 1 Hz of 40 Kepler and 24 GLONASS satellites, the whole call: 495 -> 247 us.
 // Four CTAs per SM (64 registers): with two 291 us, with three 258.
-template <int EPT>
+template <int EPT, int TS>
 __global__ void __launch_bounds__(kTileThreads, 4) k_broadcast_orbits(const pf_broadcast_t* __restrict__ recs, int n_recs,
                                    const int* __restrict__ idx, const double* __restrict__ times,
                                    int n_epoch, int n_sat, double glo_step, const double* tbl, int kc,
                                    double* __restrict__ pos, double* __restrict__ clk, int* __restrict__ err) {
-  constexpr int kE = 32 * EPT;
-  __shared__ int s_idx[kE][kTileS + 1];
-  __shared__ double s_pos[32][3 * kTileS + 1];
-  __shared__ double s_clk[32][kTileS + 1];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int st = (n_sat + kTileS - 1) / kTileS, et = (n_epoch + kE - 1) / kE;
+  constexpr int kRows = 32 * (kTileS / TS), kE = kRows * EPT;  // epochs at a time, and of the tile
+  __shared__ int s_idx[kE][TS + 1];
+  __shared__ double s_pos[kRows][3 * TS + 1];
+  __shared__ double s_clk[kRows][TS + 1];
+  const int w = (threadIdx.x >> 5) % TS, row = (threadIdx.x >> 5) / TS * 32 + (threadIdx.x & 31);
+  const int st = (n_sat + TS - 1) / TS, et = (n_epoch + kE - 1) / kE;
   // satellites slowest: GLONASS satellites, mostly at the end of the list,
   // come last and find their table ready
-  const int s0 = (int)(blockIdx.x / et) * kTileS, e0 = (int)(blockIdx.x % et) * kE;
-  const int ns = min(kTileS, n_sat - s0);
-  if (s0 >= st * kTileS) return;
-  for (int i = threadIdx.x; i < kE * kTileS; i += kTileThreads) {
-    const int e = e0 + i / kTileS, s = s0 + i % kTileS;
-    s_idx[i / kTileS][i % kTileS] = e < n_epoch && s < n_sat ? orbit_record(idx, (long)e * n_sat + s, s, n_recs) : -1;
+  const int s0 = (int)(blockIdx.x / et) * TS, e0 = (int)(blockIdx.x % et) * kE;
+  const int ns = min(TS, n_sat - s0);
+  if (s0 >= st * TS) return;
+  for (int i = threadIdx.x; i < kE * TS; i += kTileThreads) {
+    const int e = e0 + i / TS, s = s0 + i % TS;
+    s_idx[i / TS][i % TS] = e < n_epoch && s < n_sat ? orbit_record(idx, (long)e * n_sat + s, s, n_recs) : -1;
   }
   __syncthreads();
   KeplerShared sh;
   int have = -1;
   bool waited = false;
 #pragma unroll 1
-  for (int q = 0; q < EPT && e0 + 32 * q < n_epoch; ++q) {
-    const int e = e0 + 32 * q + lane, r = s_idx[32 * q + lane][w];
+  for (int q = 0; q < EPT && e0 + kRows * q < n_epoch; ++q) {
+    const int e = e0 + kRows * q + row, r = s_idx[kRows * q + row][w];
     double p[3], c;
     p[0] = p[1] = p[2] = c = nan("");
     const bool glo = r >= 0 && recs[r].system == 'R';
@@ -446,21 +455,21 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_broadcast_orbits(const pf_b
       kepler_orbit(k, sh, recs[r].system, times[e], p, &c);
     }
     __syncthreads();  // the previous rows have left
-    s_pos[lane][3 * w] = p[0];
-    s_pos[lane][3 * w + 1] = p[1];
-    s_pos[lane][3 * w + 2] = p[2];
-    s_clk[lane][w] = c;
+    s_pos[row][3 * w] = p[0];
+    s_pos[row][3 * w + 1] = p[1];
+    s_pos[row][3 * w + 2] = p[2];
+    s_clk[row][w] = c;
     __syncthreads();
-    const int rows = min(32, n_epoch - (e0 + 32 * q));
-    const long row0 = (long)(e0 + 32 * q) * n_sat + s0;
+    const int rows = min(kRows, n_epoch - (e0 + kRows * q));
+    const long row0 = (long)(e0 + kRows * q) * n_sat + s0;
     if (pos)
-      for (int i = threadIdx.x; i < rows * 3 * kTileS; i += kTileThreads) {
-        const int er = i / (3 * kTileS), k = i % (3 * kTileS);
+      for (int i = threadIdx.x; i < rows * 3 * TS; i += kTileThreads) {
+        const int er = i / (3 * TS), k = i % (3 * TS);
         if (k < 3 * ns) pos[3 * (row0 + (long)er * n_sat) + k] = s_pos[er][k];
       }
     if (clk)
-      for (int i = threadIdx.x; i < rows * kTileS; i += kTileThreads)
-        if (i % kTileS < ns) clk[row0 + (long)(i / kTileS) * n_sat + i % kTileS] = s_clk[i / kTileS][i % kTileS];
+      for (int i = threadIdx.x; i < rows * TS; i += kTileThreads)
+        if (i % TS < ns) clk[row0 + (long)(i / TS) * n_sat + i % TS] = s_clk[i / TS][i % TS];
   }
   if (tbl && !waited) orbit_pdl_wait();  // the grid ends after the table's
 }
