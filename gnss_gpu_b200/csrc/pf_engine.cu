@@ -45,6 +45,7 @@ struct pf_engine {
   FilterCtrl* ctrl_host = nullptr;  // pinned mirror of the control blocks, then the error word
   unsigned* err_host = nullptr;     // pinned copy of the device error word (inside ctrl_host's block)
   size_t ctrl_span = 0;             // bytes from the first control block to the end of the error word
+  bool in_flight = false;           // a step or an upload may still run: chooses how read_ctrl reads
   size_t obs_slot_bytes = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
@@ -408,17 +409,20 @@ int sync_and_check(pf_engine* eng) {
   // the error word rides on the same stream as the caller's reads: one sync
   CK(cudaMemcpyAsync(eng->err_host, eng->dev.err, sizeof(unsigned), cudaMemcpyDeviceToHost, eng->stream));
   CK(cudaStreamSynchronize(eng->stream));
+  eng->in_flight = false;
   return err_status(*eng->err_host);
 }
 
-// Control blocks and the error word that follows them, in one copy: up to 8 KB
-// (16 filters) by one CTA's stores into the pinned mirror, more by the copy
-// engine, which moves large blocks faster but starts later.  With rows as kernel
-// parameters and term_done: gated DD pseudorange and carrier on 200K particles
-// 230 -> 201 us an epoch, a Doppler epoch of 300K 259 -> 238, of 1M 346 -> 332.
+// Control blocks and the error word that follows them, in one copy.  Behind work in
+// flight, or ahead of a kernel of the same call, up to 8 KB (16 filters) come by one
+// CTA's stores into the pinned mirror: the stream stays with the compute engine.  On
+// an idle stream, and above 8 KB, the copy engine is faster.  us, copy / kernel: ESS
+// of a filter (nothing else in the call) 11.4 / 12.9, upload, step and results of 8
+// filters 55.3 / 48.5, of one 43.3 / 41.9, position term 33.7 / 30.0, velocity predict
+// 34.7 / 31.1.
 constexpr size_t kMirrorBytes = 8192;
-int read_ctrl(pf_engine* eng) {
-  if (eng->ctrl_span <= kMirrorBytes) {
+int read_ctrl(pf_engine* eng, bool kernel_follows = false) {
+  if (eng->ctrl_span <= kMirrorBytes && (kernel_follows || eng->in_flight)) {
     k_mirror<<<1, kThreads, 0, eng->stream>>>((const unsigned*)eng->ctrl_dev, (unsigned*)eng->ctrl_host,
                                               (int)(eng->ctrl_span / 4));
     CK(cudaGetLastError());
@@ -426,6 +430,7 @@ int read_ctrl(pf_engine* eng) {
     CK(cudaMemcpyAsync(eng->ctrl_host, eng->ctrl_dev, eng->ctrl_span, cudaMemcpyDeviceToHost, eng->stream));
   }
   CK(cudaStreamSynchronize(eng->stream));
+  eng->in_flight = false;
   return err_status(*eng->err_host);
 }
 
@@ -436,6 +441,7 @@ int term_done(pf_engine* eng, int f, bool if_clean = false) {
   k_term_done<<<1, 1, 0, eng->stream>>>(eng->ctrl_dev + f, eng->dev.err, eng->err_host, if_clean);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(eng->stream));
+  eng->in_flight = false;
   return err_status(*eng->err_host);
 }
 
@@ -820,6 +826,7 @@ int pfe_upload_obs(pf_engine_t* eng, int slot, const pf_filter_epoch_t* fe, cons
   const int F = eng->cfg.n_filters;
   int vs = validate_obs(eng, fe, sats, n_sats_total);
   if (vs != PF_OK) return vs;
+  eng->in_flight = true;
   const int b = eng->pin_cur;
   eng->pin_cur ^= 1;
   CK(cudaEventSynchronize(eng->pin_ev[b]));
@@ -841,6 +848,7 @@ int pfe_step(pf_engine_t* eng) {
     if (!eng->initialized[f]) return set_err(PF_ENOTINIT, "filter %d not initialized", f);
   if (eng->cfg.weight_mode == PF_WEIGHT_MIXTURE && !eng->mlp_set)
     return set_err(PF_ENOTINIT, "mixture likelihood: network parameters not set (pfe_set_mlp)");
+  eng->in_flight = true;
   int n = 1;
   cudaEvent_t* ev = nullptr;
   if (eng->t_slots > 0) {
@@ -929,6 +937,7 @@ int pfe_read_timing(pf_engine_t* eng, float* step_kernel_ms, float* whole_step_m
 int pfe_step_per_filter(pf_engine_t* eng) {
   clear_err();
   if (!eng) return set_err(PF_EINVAL, "null engine");
+  eng->in_flight = true;
   int n = 0;
   for (int f = 0; f < eng->cfg.n_filters; ++f) {
     if (!eng->initialized[f]) return set_err(PF_ENOTINIT, "filter %d not initialized", f);
@@ -981,6 +990,7 @@ int pfe_graph_capture(pf_engine_t* eng, int per_filter) {
 int pfe_graph_launch(pf_engine_t* eng, int n_epochs) {
   clear_err();
   if (!eng || !eng->gexec) return set_err(PF_EINVAL, "no captured graph");
+  eng->in_flight = true;
   for (int i = 0; i < n_epochs; ++i) CK(cudaGraphLaunch(eng->gexec, eng->stream));
   return PF_OK;
 }
@@ -1132,6 +1142,7 @@ int pfe_step_io(pf_engine_t* eng, const pf_filter_epoch_t* fe, const pf_sat_t* s
   dev.err_map = eng->err_host;
   if ((s = launch_epoch(eng, 0, eng->T, dev, in)) != PF_OK) return s;
   CK(cudaStreamSynchronize(eng->stream));
+  eng->in_flight = false;
   if (*(volatile unsigned*)eng->err_host) {
     CK(cudaMemcpy(eng->err_host, eng->dev.err, sizeof(unsigned), cudaMemcpyDeviceToHost));
   }
@@ -1168,6 +1179,7 @@ static int run_estimate(pf_engine_t* eng, int filter) {
   }
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(eng->stream));
+  eng->in_flight = false;
   if (*(volatile unsigned*)eng->err_host)
     CK(cudaMemcpy(eng->err_host, eng->dev.err, sizeof(unsigned), cudaMemcpyDeviceToHost));
   return err_status(*eng->err_host);
@@ -1531,7 +1543,7 @@ int pfe_add_position_term(pf_engine_t* eng, int filter, const double* refs_ecef,
   if (!eng->initialized[filter]) return set_err(PF_ENOTINIT, "filter %d not initialized", filter);
   if (!refs_ecef || K < 1 || K > kMaxPosRefs) return set_err(PF_EINVAL, "need 1..%d references", kMaxPosRefs);
   if (!(sigma > 0.0) || !isfinite(sigma)) return set_err(PF_EINVAL, "sigma must be > 0");
-  if ((s = read_ctrl(eng)) != PF_OK) return s;
+  if ((s = read_ctrl(eng, true)) != PF_OK) return s;
   const FilterCtrl& c = eng->ctrl_host[filter];
   const FilterDesc& d = eng->hdesc[filter];
   PosTerm pt;
@@ -1645,7 +1657,7 @@ int pfe_vel_init(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const double 
     if (!isfinite(v0_ecef[i])) return set_err(PF_EINVAL, "v0 not finite");
   if (!(spread_vel >= 0.0) || !isfinite(spread_vel) || !isfinite(init_sigma))
     return set_err(PF_EINVAL, "spread_vel must be finite and >= 0");
-  if ((s = read_ctrl(eng)) != PF_OK) return s;
+  if ((s = read_ctrl(eng, true)) != PF_OK) return s;
   const int n = eng->hdesc[filter].n;
   k_vel_init<<<vel_grid(eng, n, 1), kThreads, 0, eng->stream>>>(eng->dev, filter, vs->buf, v0_ecef[0], v0_ecef[1],
                                                                   v0_ecef[2], spread_vel, init_sigma * init_sigma, step);
@@ -1659,7 +1671,7 @@ int pfe_vel_follow(pf_engine_t* eng, int filter, pf_vel_state_t* vs) {
   clear_err();
   int s = vel_check(eng, filter, vs);
   if (s != PF_OK) return s;
-  if ((s = read_ctrl(eng)) != PF_OK) return s;
+  if ((s = read_ctrl(eng, true)) != PF_OK) return s;
   const FilterCtrl& c = eng->ctrl_host[filter];
   if (!c.resample_flag || c.rs_seq == vs->seq) return PF_OK;
   const int n = eng->hdesc[filter].n;
@@ -1696,7 +1708,7 @@ int pfe_vel_predict(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const doub
   if (!isfinite(dt) || !isfinite(sigma_pos) || !isfinite(sigma_vel) || !isfinite(alpha) || !isfinite(q) ||
       sigma_pos < 0.0 || sigma_vel < 0.0)
     return set_err(PF_EINVAL, "predict parameters must be finite, sigmas >= 0");
-  if ((s = read_ctrl(eng)) != PF_OK) return s;
+  if ((s = read_ctrl(eng, true)) != PF_OK) return s;
   FilterCtrl& c = eng->ctrl_host[filter];
   const FilterDesc& d = eng->hdesc[filter];
   VelPredict vp;

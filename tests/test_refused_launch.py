@@ -187,3 +187,19 @@ out["ran"], out["after"], out["again"] = fake.fake_log().decode().splitlines(), 
     before = names[:names.index(part)] if part != "fill" else []
     assert r["status"] != 0 and len(r["ran"]) == len(before)
     assert r["after"] == r["base"] and r["again"] == 0
+
+
+def test_results_behind_a_step_and_on_an_idle_stream(fake):
+    """The control blocks come by a kernel behind a step in flight, by the copy engine
+    when nothing is: the same results."""
+    r = run(fake, r"""
+res, ess = (N.FilterResult * 1)(), C.c_double(0)
+for step in (0, 1):
+    for name, read in (("results", lambda: L.pfe_read_results(h, res)), ("ess", lambda: L.pfe_get_ess(h, 0, C.byref(ess)))):
+        if step:
+            N.check(L.pfe_step(h))
+        fake.fake_clear_log()
+        out[f"{name}{step}"] = [read(), launched("k_mirror"), res[0].initialized, ess.value]
+""")
+    assert r["results0"] == [0, 0, 1, 0.0] and r["results1"] == [0, 1, 1, 40_003.0]
+    assert r["ess0"] == [0, 0, 1, 40_003.0] and r["ess1"] == [0, 1, 1, 40_003.0]
