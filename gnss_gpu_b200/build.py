@@ -71,11 +71,17 @@ def _build_lib(lib: Path, objdir: Path, extra: list, verbose: bool) -> Path:
 
 
 def build(force: bool = False, verbose: bool = False, checked: bool = True) -> Path:
-    """Build the library (and its checked variant) when a source is newer."""
+    """Build the library (and its checked variant, side by side) when a source is newer."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    jobs = []
     if force or _stale(LIB):
-        _build_lib(LIB, PKG / "_build", [], verbose)
+        jobs.append((LIB, PKG / "_build", [], verbose))
     if checked and (force or _stale(LIB_CHECKED)):
-        _build_lib(LIB_CHECKED, PKG / "_build_checked", ["-DPF_CHECKED"], verbose)
+        jobs.append((LIB_CHECKED, PKG / "_build_checked", ["-DPF_CHECKED"], verbose))
+    with ThreadPoolExecutor(max_workers=2) as ex:
+        for r in [ex.submit(_build_lib, *j) for j in jobs]:
+            r.result()
     return LIB
 
 

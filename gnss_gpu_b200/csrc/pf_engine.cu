@@ -51,9 +51,9 @@ struct pf_engine {
   cudaGraphExec_t gexec = nullptr;
   int resident[Q_COUNT];
   int epoch_resident = 0;     // co-resident CTAs of the cooperative epoch kernel
+  int inline_resident = 0;    // the same of its variant with inline records, 0: not asked yet
   bool mlp_set = false;       // mixture mode: network parameters uploaded
   int epoch_cap = 0;          // > 0: at most this many CTAs per launch of the epoch kernel (tuning)
-  size_t epoch_smem = 0;      // its dynamic shared memory
   unsigned* bar = nullptr;    // grid barrier words (count, generation, any-resample)
   ObsRow* obs_rows = nullptr; // satellites of pfe_add_3d_term
   int sm_count = 0;
@@ -331,66 +331,70 @@ int launch_resample(pf_engine* eng, int t0, int count, int* n_launch, cudaEvent_
 }
 
 // ---- cooperative epoch kernel: instantiation table, occupancy, launch
-typedef void (*EpochKernel)(EngineDev, int, int, unsigned*, const ObsInline);
-
-template <int NCLK, int WMODE>
-EpochKernel epoch_kernel_r(int resampler) {
-  return resampler == PF_RESAMPLE_SYSTEMATIC ? (EpochKernel)k_epoch<NCLK, WMODE, PF_RESAMPLE_SYSTEMATIC>
-                                             : (EpochKernel)k_epoch<NCLK, WMODE, PF_RESAMPLE_MEGOPOLIS>;
-}
-template <int NCLK>
-EpochKernel epoch_kernel_w(int wmode, int resampler) {
-  if (wmode == PF_WEIGHT_GAUSSIAN) return epoch_kernel_r<NCLK, PF_WEIGHT_GAUSSIAN>(resampler);
-  if (wmode == PF_WEIGHT_HUBER) return epoch_kernel_r<NCLK, PF_WEIGHT_HUBER>(resampler);
-  if (wmode == PF_WEIGHT_MIXTURE) return epoch_kernel_r<NCLK, PF_WEIGHT_MIXTURE>(resampler);
-  return epoch_kernel_r<NCLK, PF_WEIGHT_GENERIC>(resampler);
-}
-EpochKernel epoch_kernel(const pf_engine* eng) {
-  const int w = eng->cfg.weight_mode, r = eng->cfg.resampler;
-  switch (eng->cfg.n_clk) {
-    case 1: return epoch_kernel_w<1>(w, r);
-    case 2: return epoch_kernel_w<2>(w, r);
-    case 3: return epoch_kernel_w<3>(w, r);
-    default: return epoch_kernel_w<4>(w, r);
+template <class IN>
+struct EpochKernels {
+  typedef void (*Fn)(EngineDev, int, int, unsigned*, const IN);
+  template <int NCLK, int WMODE>
+  static Fn by_resampler(int resampler) {
+    return resampler == PF_RESAMPLE_SYSTEMATIC ? (Fn)k_epoch<NCLK, WMODE, PF_RESAMPLE_SYSTEMATIC, IN>
+                                               : (Fn)k_epoch<NCLK, WMODE, PF_RESAMPLE_MEGOPOLIS, IN>;
   }
-}
+  template <int NCLK>
+  static Fn by_weight(int wmode, int resampler) {
+    if (wmode == PF_WEIGHT_GAUSSIAN) return by_resampler<NCLK, PF_WEIGHT_GAUSSIAN>(resampler);
+    if (wmode == PF_WEIGHT_HUBER) return by_resampler<NCLK, PF_WEIGHT_HUBER>(resampler);
+    if (wmode == PF_WEIGHT_MIXTURE) return by_resampler<NCLK, PF_WEIGHT_MIXTURE>(resampler);
+    return by_resampler<NCLK, PF_WEIGHT_GENERIC>(resampler);
+  }
+  static Fn of(const pf_engine* eng) {
+    const int w = eng->cfg.weight_mode, r = eng->cfg.resampler;
+    switch (eng->cfg.n_clk) {
+      case 1: return by_weight<1>(w, r);
+      case 2: return by_weight<2>(w, r);
+      case 3: return by_weight<3>(w, r);
+      default: return by_weight<4>(w, r);
+    }
+  }
+};
 
-int prepare_epoch_kernel(pf_engine* eng) {
-  EpochKernel k = epoch_kernel(eng);
-  eng->epoch_smem = 0;  // no dynamic shared memory
-  CK(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eng->epoch_smem));
+// CTAs of an epoch kernel that are resident at once (no dynamic shared memory),
+// found before its first launch: that of the records in the ring when the engine is
+// made, that of the inline records (loading it takes milliseconds) in pfe_step_io.
+template <class IN>
+int epoch_resident(pf_engine* eng, int* out) {
+  if (*out > 0) return PF_OK;
+  const auto k = EpochKernels<IN>::of(eng);
+  CK(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, 0));
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, eng->epoch_smem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, 0));
   if (per_sm < 1) return set_err(PF_ECUDA, "epoch kernel does not fit on an SM");
-  eng->epoch_resident = per_sm * eng->sm_count;
+  *out = per_sm * eng->sm_count;
   return PF_OK;
 }
-
 // One cooperative launch over work items [t0, t0 + count): every CTA is
 // resident at once, which the grid barriers require (the driver refuses the
 // launch otherwise).
-int launch_epoch(pf_engine* eng, int t0, int count, const EngineDev& dev, const ObsInline& in) {
-  int cap = std::min(eng->epoch_resident, kMaxEpochGrid);
+template <class IN>
+int launch_epoch(pf_engine* eng, int t0, int count, const EngineDev& dev, const IN& in, int resident) {
+  int cap = std::min(resident, kMaxEpochGrid);
   if (eng->epoch_cap > 0) cap = std::min(cap, eng->epoch_cap);
   const int grid = std::max(1, std::min(count, cap));
   cudaLaunchConfig_t lc;
   memset(&lc, 0, sizeof(lc));
   lc.gridDim = dim3((unsigned)grid);
   lc.blockDim = dim3(kThreads);
-  lc.dynamicSmemBytes = eng->epoch_smem;
   lc.stream = eng->stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   lc.attrs = attr;
   lc.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&lc, epoch_kernel(eng), dev, t0, count, eng->bar, in);
+  cudaError_t e = cudaLaunchKernelEx(&lc, EpochKernels<IN>::of(eng), dev, t0, count, eng->bar, in);
   if (e != cudaSuccess) return set_err(PF_ECUDA, "k_epoch cooperative launch: %s", cudaGetErrorString(e));
   return PF_OK;
 }
 int launch_epoch(pf_engine* eng, int t0, int count) {
-  static const ObsInline none{};  // the records are in the observation ring
-  return launch_epoch(eng, t0, count, eng->dev, none);
+  return launch_epoch(eng, t0, count, eng->dev, ObsInRing{}, eng->epoch_resident);
 }
 
 bool use_chain(const pf_engine* eng) { return (eng->cfg.flags & PF_FLAG_KERNEL_CHAIN) != 0; }
@@ -613,7 +617,7 @@ int pfe_create(const pf_engine_config_t* cfg, const pf_filter_params_t* filters,
   if ((st = occupancy(k_offs, eng->sm_count, &eng->resident[Q_OFFS])) != PF_OK) return fail(st);
   if ((st = occupancy(k_merge, eng->sm_count, &eng->resident[Q_MERGE])) != PF_OK) return fail(st);
   if ((st = occupancy(k_mego, eng->sm_count, &eng->resident[Q_MEGO])) != PF_OK) return fail(st);
-  if ((st = prepare_epoch_kernel(eng)) != PF_OK) return fail(st);
+  if ((st = epoch_resident<ObsInRing>(eng, &eng->epoch_resident)) != PF_OK) return fail(st);
   if ((st = occupancy(k_init<7>, eng->sm_count, &eng->resident[Q_INIT])) != PF_OK) return fail(st);
   if ((st = occupancy(k_estimate<7>, eng->sm_count, &eng->resident[Q_EST])) != PF_OK) return fail(st);
   if ((st = occupancy(k_export<7>, eng->sm_count, &eng->resident[Q_EXPORT])) != PF_OK) return fail(st);
@@ -1126,6 +1130,7 @@ int pfe_step_io(pf_engine_t* eng, const pf_filter_epoch_t* fe, const pf_sat_t* s
   in.bytes = 0;
   unsigned char* h = in.data;
   if (bytes <= sizeof(in.data)) {
+    if ((s = epoch_resident<ObsInline>(eng, &eng->inline_resident)) != PF_OK) return s;
     in.bytes = (int)bytes;
   } else {
     const int b = eng->pin_cur;
@@ -1140,7 +1145,9 @@ int pfe_step_io(pf_engine_t* eng, const pf_filter_epoch_t* fe, const pf_sat_t* s
   EngineDev dev = eng->dev;
   dev.ctrl_map = eng->ctrl_host;
   dev.err_map = eng->err_host;
-  if ((s = launch_epoch(eng, 0, eng->T, dev, in)) != PF_OK) return s;
+  s = in.bytes ? launch_epoch(eng, 0, eng->T, dev, in, eng->inline_resident)
+               : launch_epoch(eng, 0, eng->T, dev, ObsInRing{}, eng->epoch_resident);
+  if (s != PF_OK) return s;
   CK(cudaStreamSynchronize(eng->stream));
   eng->in_flight = false;
   if (*(volatile unsigned*)eng->err_host) {

@@ -33,6 +33,8 @@
 // (the epoch just wrote them).  Phase 4 needs no CTA barrier per tile: warps
 // work on independent segments.
 #pragma once
+#include <type_traits>
+
 #include "pf_engine_kernels.cuh"
 #include "pf_learned.cuh"
 #include "pf_generic.cuh"
@@ -430,9 +432,9 @@ __device__ __forceinline__ void merge_rows(const EngineDev& e, int t, int j, con
 #ifndef PF_EPOCH_MINB
 #define PF_EPOCH_MINB 2  // resident CTAs per SM the epoch kernel is compiled for
 #endif
-template <int NCLK, int WMODE, int RESAMPLER>
+template <int NCLK, int WMODE, int RESAMPLER, class IN>
 __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, int t0, int count, unsigned* bar,
-                                                                     const __grid_constant__ ObsInline in) {
+                                                                     const __grid_constant__ IN in) {
   constexpr int D = 3 + NCLK;
   constexpr int NV = 2 + D + 6;
   constexpr int kWarps = kThreads / 32;
@@ -457,11 +459,14 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
   unsigned gen = ld_relaxed(bar + 1);
   if (threadIdx.x == 0) s_dec_f = -1;
   if (threadIdx.x < kRowBufs) s_rows[threadIdx.x] = s_merged[threadIdx.x] = 0u;  // ordered by the first table's barriers
-  const unsigned char* const obs0 = in.bytes > 0 ? in.data : e.obs;
-  if (in.bytes > 0 && blockIdx.x == gridDim.x - 1)  // slot 0 keeps them for a later step without an upload
-    for (int i = threadIdx.x * 8; i < in.bytes; i += kThreads * 8)
-      *reinterpret_cast<unsigned long long*>(const_cast<unsigned char*>(e.obs) + i) =
-          *reinterpret_cast<const unsigned long long*>(in.data + i);
+  const unsigned char* obs0 = e.obs;
+  if constexpr (std::is_same<IN, ObsInline>::value) {
+    obs0 = in.data;
+    if (blockIdx.x == gridDim.x - 1)  // slot 0 keeps them for a later step without an upload
+      for (int i = threadIdx.x * 8; i < in.bytes; i += kThreads * 8)
+        *reinterpret_cast<unsigned long long*>(const_cast<unsigned char*>(e.obs) + i) =
+            *reinterpret_cast<const unsigned long long*>(in.data + i);
+  }
   int cb, ce;
   weighted_chunk<NCLK, WMODE>(e, t0, count, obs0, s_u64, s_cut, cb, ce);
 

@@ -203,3 +203,17 @@ for step in (0, 1):
 """)
     assert r["results0"] == [0, 0, 1, 0.0] and r["results1"] == [0, 1, 1, 40_003.0]
     assert r["ess0"] == [0, 0, 1, 40_003.0] and r["ess1"] == [0, 1, 1, 40_003.0]
+
+
+def test_only_the_one_call_step_carries_its_records(fake):
+    """A step whose records are in the ring launches the kernel without the 3.7 KB
+    parameter; the one-call step takes it where the records fit."""
+    r = run(fake, r"""
+fe, sats = np.zeros(1, N.FILTER_EPOCH_DTYPE), np.zeros(16, N.SAT_DTYPE)
+res = (N.FilterResult * 1)()
+for name, call in (("step", lambda: L.pfe_step(h)), ("per_filter", lambda: L.pfe_step_per_filter(h)),
+                   ("io", lambda: L.pfe_step_io(h, N.vptr(fe), N.vptr(sats), 16, res))):
+    fake.fake_clear_log()
+    out[name] = [call(), launched("k_epoch"), launched("ObsInRing"), launched("ObsInline")]
+""")
+    assert r["step"] == r["per_filter"] == [0, 1, 1, 0] and r["io"] == [0, 1, 0, 1]
