@@ -749,16 +749,18 @@ int pf_broadcast_orbits(const pf_broadcast_t* d_recs, int n_recs, const int* d_r
   int dev = 0, sms = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // tiles of one satellite or of eight (kNarrowSats), of four epochs per thread
-  // once that still gives every SM its four CTAs
-  const bool narrow = n_sat <= kNarrowSats;
-  const int ts = narrow ? 1 : kTileS, rows = 32 * kTileS / ts;
+  // tiles of one satellite (kNarrowSats), of eight, or of 256 (wide_tiles); the first
+  // two of four epochs per thread once that still gives every SM its four CTAs
+  const bool narrow = n_sat <= kNarrowSats, wide = wide_tiles(n_epoch, n_sat);
+  const int ts = narrow ? 1 : wide ? kTileThreads : kTileS, rows = kTileThreads / ts;
   const long cols = (n_sat + ts - 1) / ts, tiles = cols * (((long)n_epoch + rows - 1) / rows);
-  const bool four = tiles >= 4l * sms * 4;
+  const bool four = !wide && tiles >= 4l * sms * 4;
   const unsigned grid = (unsigned)(four ? cols * (((long)n_epoch + 4 * rows - 1) / (4 * rows)) : tiles);
-  const auto orbits = narrow ? (four ? k_broadcast_orbits<4, 1> : k_broadcast_orbits<1, 1>)
-                             : (four ? k_broadcast_orbits<4, kTileS> : k_broadcast_orbits<1, kTileS>);
-  const long need_cols = (n_sat + kTileS - 1) / kTileS;
+  const auto orbits = wide     ? k_broadcast_orbits<1, kTileThreads>
+                      : narrow ? (four ? k_broadcast_orbits<4, 1> : k_broadcast_orbits<1, 1>)
+                               : (four ? k_broadcast_orbits<4, kTileS> : k_broadcast_orbits<1, kTileS>);
+  const auto glo_need = wide ? k_glo_need<true> : k_glo_need<false>;
+  const long need = wide ? cols : (long)((n_sat + kTileS - 1) / kTileS) * (((long)n_epoch + kNeedE - 1) / kNeedE);
   // GLONASS state table: the epochs of a record share its states at whole
   // steps from toe, so they are integrated once per (record, direction)
   int kc = 0;
@@ -784,8 +786,8 @@ int pf_broadcast_orbits(const pf_broadcast_t* d_recs, int n_recs, const int* d_r
   double* tbl = (double*)(scratch + kmax_bytes);
   cudaError_t ce = cudaMemsetAsync(kmax, 0, kmax_bytes, st);
   if (ce == cudaSuccess) {
-    k_glo_need<<<(unsigned)(need_cols * (((long)n_epoch + kNeedE - 1) / kNeedE)), kTileThreads, 0, st>>>(
-        d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step, kc, kmax);
+    glo_need<<<(unsigned)need, kTileThreads, 0, st>>>(d_recs, n_recs, d_rec_index, d_times, n_epoch, n_sat, glo_step,
+                                                      kc, kmax);
     ce = cudaGetLastError();
   }
   cudaLaunchConfig_t lc;

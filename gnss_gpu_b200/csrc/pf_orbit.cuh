@@ -329,6 +329,18 @@ constexpr int kTileThreads = 32 * kTileS;
 // 86,400 46 (53)) and of the other tile where GLONASS rows are short (7 x 20,000 109
 // / 141).
 constexpr int kNarrowSats = 4;
+// Few epochs of very many satellites leave most lanes of those tiles without an epoch:
+// there a tile is one epoch of 256 satellites, a lane per satellite, and so is a warp
+// of k_glo_need.  Whole calls, us, tiles of eight / of 256 (and one thread per
+// satellite-epoch, before the tiles): Kepler 1 epoch x 8,192 26 / 22 (25), 1 x 100,000
+// 194 / 24 (26), 8 x 16,384 37 / 22 (30), 28 x 28,672 71 / 61 (77), 28 x 100,000 219 /
+// 182 (218); GLONASS 1 x 100,000 536 / 87 (98), 16 x 50,000 172 / 123 (287).  With fewer
+// satellites per epoch the tiles of eight are level or ahead, as GLONASS and Kepler
+// records side by side keep a warp of 256's on both paths: 5 x GPS to 3 x GLONASS, 16 x
+// 8,192 38 / 47, 16 x 16,384 47 / 49, 16 x 28,672 90 / 72.
+inline bool wide_tiles(int n_epoch, int n_sat) {
+  return n_epoch <= 28 && n_sat >= 8192 && n_sat >= 1024ll * n_epoch;
+}
 
 // Programmatic dependent launch: the state table is needed by GLONASS tiles
 // only, so the orbit kernel starts while the table is made.  What the previous
@@ -344,19 +356,21 @@ __device__ inline void orbit_pdl_wait() { asm volatile("griddepcontrol.wait;" ::
 // satellite through kNeedE / 32 epochs and raises the count of a record when it
 // leaves it (an atomic per satellite-epoch took 150 us on a day of 24 satellites).
 constexpr int kNeedE = 512;
+template <bool WIDE>
 __global__ void __launch_bounds__(kTileThreads) k_glo_need(const pf_broadcast_t* __restrict__ recs, int n_recs,
                            const int* __restrict__ idx, const double* __restrict__ times, int n_epoch, int n_sat,
                            double step, int kc, int* __restrict__ kmax) {
   orbit_pdl_trigger();
-  const int st = (n_sat + kTileS - 1) / kTileS;
-  const int s = (int)(blockIdx.x % st) * kTileS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (s >= n_sat) return;  // whole warps
-  const int e0 = (int)(blockIdx.x / st) * kNeedE, e1 = min(n_epoch, e0 + kNeedE);
+  const int lane = threadIdx.x & 31, st = (n_sat + kTileS - 1) / kTileS;
+  const int s = WIDE ? (int)blockIdx.x * kTileThreads + threadIdx.x
+                     : (int)(blockIdx.x % st) * kTileS + (threadIdx.x >> 5);
+  const int e0 = WIDE ? 0 : (int)(blockIdx.x / st) * kNeedE;
+  const int e1 = s >= n_sat ? e0 : WIDE ? n_epoch : min(n_epoch, e0 + kNeedE);
   int slot = -1, need = 0;
   auto raise = [&](int sl, int m) {
     if (*(volatile int*)(kmax + sl) < m) atomicMax(kmax + sl, m);
   };
-  for (int e = e0 + lane; e < e1; e += 32) {
+  for (int e = WIDE ? e0 : e0 + lane; e < e1; e += WIDE ? 1 : 32) {
     const int r = orbit_record(idx, (long)e * n_sat + s, s, n_recs);
     if (r < 0 || recs[r].system != 'R') continue;
     const double el = wrap_half_week(broadcast_rx_sow('R', times[e]) - recs[r].u.glonass.toe);
@@ -412,11 +426,13 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_broadcast_orbits(const pf_b
                                    const int* __restrict__ idx, const double* __restrict__ times,
                                    int n_epoch, int n_sat, double glo_step, const double* tbl, int kc,
                                    double* __restrict__ pos, double* __restrict__ clk, int* __restrict__ err) {
-  constexpr int kRows = 32 * (kTileS / TS), kE = kRows * EPT;  // epochs at a time, and of the tile
+  constexpr bool kWide = TS == kTileThreads;  // lanes along the satellites of one epoch
+  constexpr int kRows = kTileThreads / TS, kE = kRows * EPT;  // epochs at a time, and of the tile
   __shared__ int s_idx[kE][TS + 1];
   __shared__ double s_pos[kRows][3 * TS + 1];
   __shared__ double s_clk[kRows][TS + 1];
-  const int w = (threadIdx.x >> 5) % TS, row = (threadIdx.x >> 5) / TS * 32 + (threadIdx.x & 31);
+  const int w = kWide ? threadIdx.x : (threadIdx.x >> 5) % TS;
+  const int row = kWide ? 0 : (threadIdx.x >> 5) / TS * 32 + (threadIdx.x & 31);
   const int st = (n_sat + TS - 1) / TS, et = (n_epoch + kE - 1) / kE;
   // satellites slowest: GLONASS satellites, mostly at the end of the list,
   // come last and find their table ready
