@@ -1674,11 +1674,11 @@ int pfe_vel_init(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const double 
   return sync_and_check(eng);
 }
 
-int pfe_vel_follow(pf_engine_t* eng, int filter, pf_vel_state_t* vs) {
+static int vel_follow(pf_engine* eng, int filter, pf_vel_state_t* vs, bool kernel_follows) {
   clear_err();
   int s = vel_check(eng, filter, vs);
   if (s != PF_OK) return s;
-  if ((s = read_ctrl(eng, true)) != PF_OK) return s;
+  if ((s = read_ctrl(eng, kernel_follows)) != PF_OK) return s;
   const FilterCtrl& c = eng->ctrl_host[filter];
   if (!c.resample_flag || c.rs_seq == vs->seq) return PF_OK;
   const int n = eng->hdesc[filter].n;
@@ -1690,6 +1690,9 @@ int pfe_vel_follow(pf_engine_t* eng, int filter, pf_vel_state_t* vs) {
   vs->seq = c.rs_seq;
   return sync_and_check(eng);
 }
+
+// Mostly nothing is pending, and the read is all there is to the call.
+int pfe_vel_follow(pf_engine_t* eng, int filter, pf_vel_state_t* vs) { return vel_follow(eng, filter, vs, false); }
 
 }  // extern "C"
 
@@ -1756,7 +1759,7 @@ int pfe_vel_predict(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const doub
 int pfe_vel_doppler(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const pf_doppler_row_t* rows, int n_rows,
                     double wavelength, double sigma_mps, double gain, double max_update, int kf) {
   clear_err();
-  int s = pfe_vel_follow(eng, filter, vs);
+  int s = vel_follow(eng, filter, vs, true);
   if (s != PF_OK) return s;
   if (n_rows < 1 || n_rows > kMaxDopplerRows || !rows) return set_err(PF_ECAP, "need 1..%d rows", kMaxDopplerRows);
   if (!(wavelength > 0.0) || !isfinite(wavelength) || !(sigma_mps > 0.0) || !isfinite(sigma_mps) || !isfinite(gain) ||

@@ -217,3 +217,19 @@ for name, call in (("step", lambda: L.pfe_step(h)), ("per_filter", lambda: L.pfe
     out[name] = [call(), launched("k_epoch"), launched("ObsInRing"), launched("ObsInline")]
 """)
     assert r["step"] == r["per_filter"] == [0, 1, 1, 0] and r["io"] == [0, 1, 0, 1]
+
+
+def test_velocities_with_nothing_to_follow_are_read_by_the_copy_engine(fake):
+    """Nothing follows the read of an idle engine's control blocks, so it is a copy;
+    the Doppler update's own kernels follow it."""
+    r = run(fake, r"""
+vs, v0, row = N.VelState(), np.zeros(3), np.zeros(1, N.DOPPLER_ROW_DTYPE)
+vs.buf = block(2 * 12 * n * 8)
+row["sat"], row["weight"] = 2e7, 1.0
+N.check(L.pfe_vel_init(h, 0, C.byref(vs), N.dptr(v0), 0.1, 1.0, 0))
+for name, call in (("follow", lambda: L.pfe_vel_follow(h, 0, C.byref(vs))),
+                   ("doppler", lambda: L.pfe_vel_doppler(h, 0, C.byref(vs), N.vptr(row), 1, 0.19, 0.5, 0.0, 0.0, 0))):
+    fake.fake_clear_log()
+    out[name] = [call(), launched("k_mirror"), launched("k_doppler")]
+""")
+    assert r["follow"] == [0, 0, 0] and r["doppler"] == [0, 1, 1]
