@@ -136,13 +136,25 @@ __device__ __forceinline__ void cta_chunk(int t0, int count, int& b, int& e) {
 // (draws, statistics, CDF) over one satellite, fitted to phase 1 of 48 x 100K
 // filters with 8 to 40 satellites (per tile, one clock, us: Gaussian 4.3 + 0.084
 // s, Huber 4.1 + 0.114 s, mixture 4.4 + 0.27 s).  256 filters with 6 to 40
-// satellites: phase 1 ended between 88 and 178 us with equal numbers.
+// satellites: phase 1 ended between 88 and 178 us with equal numbers.  With several
+// clocks the same times 8 / 5, chosen between 5 / 5 and 12 / 5 (256 x 20K Huber filters
+// of 4 clocks 248 us; 260 and 249 us; the Gaussian ones 213; 215 and 217).
+//
+// The cut itself is three dependent loads per filter and a scan, 3 us for 256
+// filters, 8 for 1024 and 40 for 4096, and a chunk of many small filters has about the average
+// satellites anyway: below kCutTiles tiles per filter the numbers are equal.  Epoch
+// kernel, us, cut by cost / by number: Huber, 6 to 40 satellites, 64 x 15 tiles
+// 56 / 64, 256 x 20 204 / 225, 256 x 10 116 / 123, 1024 x 12 471 / 492, 1024 x 6 266 /
+// 267 (Gaussian 224 / 222, mixture 351 / 363), 1024 x 3 167 / 163, 256 x 5 70 / 72
+// (Gaussian 64 / 62, mixture 97 / 94), 4096 x 1 227 / 183; with satellites equal
+// throughout the cut costs up to 3 % of the kernel (64 x 30 tiles 106 / 102).
+constexpr int kCutTiles = 8;
 template <int NCLK, int WMODE>
 __device__ __forceinline__ void weighted_chunk(const EngineDev& e, int t0, int count, const unsigned char* obs0,
                                                unsigned long long* s_u64, int* s_cut, int& cb, int& ce) {
   constexpr int kFix = (WMODE == PF_WEIGHT_GAUSSIAN ? 48 : WMODE == PF_WEIGHT_MIXTURE ? 22 : 34) * (NCLK > 1 ? 8 : 5) / 5;
   const int f0 = __ldg(e.tile_filter + t0), nf = __ldg(e.tile_filter + t0 + count - 1) - f0 + 1;
-  if (nf == 1 || count <= (int)gridDim.x) {  // CTA-uniform
+  if (count <= (int)gridDim.x || nf == 1 || count < kCutTiles * nf) {  // CTA-uniform; the first needs no load
     cta_chunk(t0, count, cb, ce);
     return;
   }
