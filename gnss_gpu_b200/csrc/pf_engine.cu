@@ -1625,7 +1625,6 @@ int pfe_add_obs_term(pf_engine_t* eng, int filter, int kind, const pf_obs_row_t*
   ObsBlock b;
   memset(&b, 0, sizeof(b));
   b.n = n_rows;
-  b.kind = kind;
   b.accumulate = accumulate ? 1 : 0;
   b.gate_min = std::min(n_rows, 3);
   b.inv_sigma2 = 1.0 / (sigma * sigma);
@@ -1650,8 +1649,8 @@ static int vel_check(pf_engine_t* eng, int filter, pf_vel_state_t* vs) {
   return PF_OK;
 }
 
-static int vel_grid(pf_engine_t* eng, int n, int per_thread) {
-  return std::max(1, std::min(eng->sm_count * 8, (n + kThreads * per_thread - 1) / (kThreads * per_thread)));
+static int vel_grid(pf_engine_t* eng, int n) {
+  return std::max(1, std::min(eng->sm_count * 8, (n + kThreads - 1) / kThreads));
 }
 
 int pfe_vel_init(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const double v0_ecef[3], double spread_vel,
@@ -1666,7 +1665,7 @@ int pfe_vel_init(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const double 
     return set_err(PF_EINVAL, "spread_vel must be finite and >= 0");
   if ((s = read_ctrl(eng, true)) != PF_OK) return s;
   const int n = eng->hdesc[filter].n;
-  k_vel_init<<<vel_grid(eng, n, 1), kThreads, 0, eng->stream>>>(eng->dev, filter, vs->buf, v0_ecef[0], v0_ecef[1],
+  k_vel_init<<<vel_grid(eng, n), kThreads, 0, eng->stream>>>(eng->dev, filter, vs->buf, v0_ecef[0], v0_ecef[1],
                                                                   v0_ecef[2], spread_vel, init_sigma * init_sigma, step);
   CK(cudaGetLastError());
   vs->sel = 0;
@@ -1684,7 +1683,7 @@ static int vel_follow(pf_engine* eng, int filter, pf_vel_state_t* vs, bool kerne
   const int n = eng->hdesc[filter].n;
   const double* in = vs->buf + (size_t)vs->sel * kVelComp * n;
   double* out = vs->buf + (size_t)(vs->sel ^ 1) * kVelComp * n;
-  k_vel_gather<<<vel_grid(eng, n, 1), kThreads, 0, eng->stream>>>(eng->dev, filter, in, out);
+  k_vel_gather<<<vel_grid(eng, n), kThreads, 0, eng->stream>>>(eng->dev, filter, in, out);
   CK(cudaGetLastError());
   vs->sel ^= 1;
   vs->seq = c.rs_seq;
@@ -1783,7 +1782,6 @@ int pfe_vel_doppler(pf_engine_t* eng, int filter, pf_vel_state_t* vs, const pf_d
   DopplerArgs a;
   memset(&a, 0, sizeof(a));
   a.n_sat = n_rows;
-  a.kf = kf ? 1 : 0;
   a.wavelength = wavelength;
   a.sigma = sigma_mps;
   a.gain = gain;

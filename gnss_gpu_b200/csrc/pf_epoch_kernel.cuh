@@ -9,8 +9,9 @@
 //      measured faster than staging them through shared memory with
 //      cp.async).  Systematic: also the segment and tile levels of the
 //      tiled integer CDF -- each warp quantises its 128 particles against
-//      its own maximum and stores their prefixes inside the segment, warp 0
-//      rescales the segment sums exactly to the tile maximum.
+//      its own maximum and stores their prefixes inside the segment, and the
+//      warp that merges the tile's rows (the warps take turns, two tiles
+//      behind) rescales the segment sums exactly to the tile maximum.
 //   -- barrier
 //   2  per-filter merge of the tile rows (filter f_first + j by CTA j mod G):
 //      ESS, weighted mean / covariance, device-side resample decision.
@@ -141,13 +142,14 @@ __device__ __forceinline__ void cta_chunk(int t0, int count, int& b, int& e) {
 // of 4 clocks 248 us; 260 and 249 us; the Gaussian ones 213; 215 and 217).
 //
 // The cut itself is three dependent loads per filter and a scan, 3 us for 256
-// filters, 8 for 1024 and 40 for 4096, and a chunk of many small filters has about the average
-// satellites anyway: below kCutTiles tiles per filter the numbers are equal.  Epoch
-// kernel, us, cut by cost / by number: Huber, 6 to 40 satellites, 64 x 15 tiles
-// 56 / 64, 256 x 20 204 / 225, 256 x 10 116 / 123, 1024 x 12 471 / 492, 1024 x 6 266 /
-// 267 (Gaussian 224 / 222, mixture 351 / 363), 1024 x 3 167 / 163, 256 x 5 70 / 72
-// (Gaussian 64 / 62, mixture 97 / 94), 4096 x 1 227 / 183; with satellites equal
-// throughout the cut costs up to 3 % of the kernel (64 x 30 tiles 106 / 102).
+// filters, 8 for 1024 and 40 for 4096, and a chunk of many small filters has about
+// the average satellites anyway: below kCutTiles tiles per filter the numbers are
+// equal.  Epoch kernel, us, cut by cost / by number: Huber, 6 to 40 satellites,
+// 64 x 15 tiles 56 / 64, 256 x 20 204 / 225, 256 x 10 116 / 123, 1024 x 12 471 / 492,
+// 1024 x 6 266 / 267 (Gaussian 224 / 222, mixture 351 / 363), 1024 x 3 167 / 163,
+// 256 x 5 70 / 72 (Gaussian 64 / 62, mixture 97 / 94), 4096 x 1 227 / 183; with
+// satellites equal throughout the cut costs up to 3 % of the kernel (64 x 30 tiles
+// 106 / 102).
 constexpr int kCutTiles = 8;
 template <int NCLK, int WMODE>
 __device__ __forceinline__ void weighted_chunk(const EngineDev& e, int t0, int count, const unsigned char* obs0,
@@ -681,7 +683,7 @@ __global__ void __launch_bounds__(kThreads, PF_EPOCH_MINB) k_epoch(EngineDev e, 
         if (p0 + k >= n) lwv[k] = -INFINITY;
     }
 
-    // per-warp statistics, then warp 0 merges the warp rows into the tile row
+    // per-warp statistics, then one warp merges the warp rows into the tile row
     {
       float wm = fmaxf(fmaxf(lwv[0], lwv[1]), fmaxf(lwv[2], lwv[3]));
       wm = warp_max(wm);

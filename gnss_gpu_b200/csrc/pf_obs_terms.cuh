@@ -42,7 +42,6 @@ struct ObsRowsIn {
 
 struct ObsBlock {
   int n;
-  int kind;
   int accumulate;   // 1: add to the current log-weights, 0: overwrite them
   int gate_min;     // rows that must stay inside the gate
   double inv_sigma2;

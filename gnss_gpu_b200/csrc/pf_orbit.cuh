@@ -13,9 +13,10 @@
 //  * Sagnac: rotation of the satellite about the earth axis by the signal
 //    transit time (python/gnss_gpu/range_model.py:12-40).
 //
-// One thread per (epoch, satellite); FP64 throughout.  The work is O(S) per
-// epoch and tiny next to the filter step, so the kernels are written for
-// batching many epochs into one launch, not for bandwidth.
+// FP64 throughout.  The work is O(S) per epoch and small next to the filter step, so
+// the kernels batch many epochs into one launch: the broadcast orbits in tiles of
+// epochs x satellites (kTileS, kNarrowSats, wide_tiles), the others with a thread per
+// (epoch, satellite).
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -240,12 +241,12 @@ __device__ inline void glo_rk4(double h, double* x, const double* acc) {
 }
 
 // Full steps of the GLONASS integration of a record at GPST second of
-// week t and what is left for the residual step: the loop of
-// orbit_glonass.py:122-150 without the arithmetic (rem decremented in the
-// same order, so it is bit-identical).  Returns false past kGloMaxSteps.
+// week t and what is left for the residual step: what the loop of
+// orbit_glonass.py:122-150 leaves, bit for bit.  Returns false past kGloMaxSteps.
 //
-// With a whole number of seconds per step every difference is exact (it lies
-// on the grid of el's last bit), so the count is a quotient.
+// With a whole number of seconds per step every difference of the loop is exact (it
+// lies on the grid of el's last bit), so the count is a quotient; otherwise the
+// loop runs, without its arithmetic (rem decremented in the same order).
 __device__ inline bool glo_plan(const pf_glonass_state_t& g, double t, double step, double& el, double& base,
                                 long& k, double& rem) {
   el = wrap_half_week(broadcast_rx_sow('R', t) - g.toe);

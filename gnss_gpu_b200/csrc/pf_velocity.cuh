@@ -205,7 +205,6 @@ __device__ __forceinline__ void particle_ecef(const FilterDesc* fd, const Filter
 
 struct DopplerArgs {
   int n_sat;
-  int kf;           // 1: velocity Kalman update (pf_device.cu:750-887)
   double wavelength, sigma, gain, max_update;
 };
 
